@@ -109,9 +109,11 @@ struct pw_ctx {
   pwb::DevBuf ekin;             // T [n2][n1][n0]  |G|^2/2 on the full coarse spectrum
   pwb::DevBuf teter;            // T [n2][n1][n0]
   pwb::DevBuf vtot;             // T [N_fine]
-  pwb::DevBuf vperm;            // T: vtot in the lane order of the fused fine-plane kernel's
-                                //    row pass (fft_variant 2), rebuilt whenever vtot is written
+  pwb::DevBuf vtot_t;           // T: vtot with its planes transposed ([z][x][y]), sphere-cut contexts;
+                                //    rebuilt whenever vtot is written
   pwb::DevBuf tw[6];            // complex T twiddles for n0,n1,n2,nf0,nf1,nf2
+  // spectrum tables in the [kz][kx][ky] order of the register-transform kernels
+  pwb::DevBuf ekin_t, teter_t, wmask_t, exx_kern_t, ekin_k_t, ekin_kb_t;
   bool have_vtot = false;
   bool have_nl = false;
   pwb::NonlocalDev nl;
@@ -262,6 +264,9 @@ struct Launch {
     }
   }
 };
+
+// a coarse-spectrum table from the host: [kz][ky][kx] into dst and [kz][kx][ky] into dst_t
+int upload_spectrum(pw_ctx* c, DevBuf& dst, DevBuf& dst_t, const double* src);
 
 // exact exchange of sphere-cut (G-space) FP64 contexts (gs_exx.cu)
 int gs_exx_setup(pw_ctx* c, double frac, double mu, int divergence_type, double ecut);

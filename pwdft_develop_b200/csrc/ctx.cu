@@ -59,14 +59,40 @@ int upload_real(pw_ctx* c, DevBuf& dst, const double* src, size_t n) {
   return PW_OK;
 }
 
-// the fine-plane kernel's permuted copy of vtot, rebuilt after every write of
-// vtot (on the legacy stream, finished before returning, so that streams and
+// [z][y][x] -> [z][x][y], 32 x 32 tiles
+template <typename T> static __global__ void k_table_t(const T* __restrict__ src, T* __restrict__ dst, int n0, int n1) {
+  __shared__ T tile[32][33];
+  const long o = (long)blockIdx.z * n0 * n1;
+  const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, tx = threadIdx.x;
+  for (int i = threadIdx.y; i < 32; i += blockDim.y)
+    if (y0 + i < n1 && x0 + tx < n0) tile[i][tx] = src[o + (long)(y0 + i) * n0 + x0 + tx];
+  __syncthreads();
+  for (int i = threadIdx.y; i < 32; i += blockDim.y)
+    if (x0 + i < n0 && y0 + tx < n1) dst[o + (long)(x0 + i) * n1 + y0 + tx] = tile[tx][i];
+}
+static int planes_t(pw_ctx* c, const void* src, void* dst, const int n[3]) {
+  const dim3 g((n[0] + 31) / 32, (n[1] + 31) / 32, n[2]), b(32, 8);
+  if (c->prec == PW_F64) k_table_t<double><<<g, b>>>((const double*)src, (double*)dst, n[0], n[1]);
+  else k_table_t<float><<<g, b>>>((const float*)src, (float*)dst, n[0], n[1]);
+  PWB_CUDA(cudaGetLastError());
+  PWB_CUDA(cudaStreamSynchronize(nullptr));
+  return PW_OK;
+}
+
+int upload_spectrum(pw_ctx* c, DevBuf& dst, DevBuf& dst_t, const double* src) {
+  int rc = upload_real(c, dst, src, c->ntot);
+  if (rc || (rc = dst_t.alloc((size_t)c->ntot * c->esz))) return rc;
+  return planes_t(c, dst.p, dst_t.p, c->n);
+}
+
+// the fine-plane kernel's transposed copy of vtot (sphere-cut contexts), rebuilt
+// after every write of vtot (on the legacy stream, finished before returning, so that streams and
 // graph replays that read it afterwards see the new potential)
-int refresh_vperm(pw_ctx* c) {
-  const GridEntry* g = find_grid(c->n);
-  if (!g || !c->vtot.p) return PW_OK;
-  int rc = g->vperm[c->prec == PW_F32 ? 1 : 0](c, nullptr);
-  if (rc) return rc;
+int refresh_vtot_t(pw_ctx* c) {
+  if (c->gs && c->vtot.p) {
+    int rc = c->vtot_t.alloc((size_t)c->ntotf * c->esz);
+    return rc ? rc : planes_t(c, c->vtot.p, c->vtot_t.p, c->nf);
+  }
   PWB_CUDA(cudaStreamSynchronize(nullptr));
   return PW_OK;
 }
@@ -235,8 +261,8 @@ int pw_ctx_create(const double length[3], const int numGrid[3], const int numGri
         te[idx] = b / (b + 16.0 * std::pow(a, 4.0));
       }
   int rc;
-  if ((rc = upload_real(c, c->ekin, ek.data(), ek.size())) ||
-      (rc = upload_real(c, c->teter, te.data(), te.size()))) {
+  if ((rc = upload_spectrum(c, c->ekin, c->ekin_t, ek.data())) ||
+      (rc = upload_spectrum(c, c->teter, c->teter_t, te.data()))) {
     delete c;
     return rc;
   }
@@ -311,7 +337,7 @@ int pw_set_vtot(pw_ctx* ctx, const double* vtot) {
   PWB_CHECK(ctx && vtot, PW_EINVAL, "null argument");
   PWB_CUDA(cudaSetDevice(ctx->device));
   int rc = upload_real(ctx, ctx->vtot, vtot, ctx->ntotf);
-  if (rc || (rc = refresh_vperm(ctx))) return rc;
+  if (rc || (rc = refresh_vtot_t(ctx))) return rc;
   ctx->h_vtot.assign(vtot, vtot + ctx->ntotf);
   ctx->have_vtot = true;
   return PW_OK;
@@ -596,7 +622,7 @@ int pw_set_wfn_filter(pw_ctx* ctx, int enable, double ecut) {
                        g2 = 2 * M_PI / ctx->L[2] * m2;
           m[i + (long)n0 * (j + (long)n1 * k)] = (g0 * g0 + g1 * g1 + g2 * g2) / 2 > ecut ? 0.0 : 1.0;
         }
-    int rc = upload_real(ctx, ctx->wmask, m.data(), m.size());
+    int rc = upload_spectrum(ctx, ctx->wmask, ctx->wmask_t, m.data());
     if (rc) return rc;
   }
   ctx->wfn_ecut = ecut;

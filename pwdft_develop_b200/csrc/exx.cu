@@ -122,7 +122,7 @@ int pw_exx_setup(pw_ctx* ctx, double exx_fraction, double screen_mu, int diverge
       if (mu > 0.0) k[i] += M_PI / (mu * mu);
     }
   }
-  int rc = upload_real(ctx, ctx->exx_kern, k.data(), nt);
+  int rc = upload_spectrum(ctx, ctx->exx_kern, ctx->exx_kern_t, k.data());
   if (rc) return rc;
   ctx->exx_frac = exx_fraction;
   ctx->exx_mu = mu;

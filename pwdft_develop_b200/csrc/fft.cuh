@@ -62,23 +62,9 @@ template <int R, int M, int DIR, typename V> __device__ __forceinline__ V twmul(
   }
 }
 
-// p[k] = w^k for k = 1 .. R-1 (even k: the square of w^{k/2}, odd k: w^{k-1} w),
-// each power at most about 2 log2(R) rounded products from w
-template <int R, typename V> __device__ __forceinline__ void twiddle_powers(V w, V* p) {
-  p[1] = w;
-  sfor<2, R>([&](auto kI) {
-    constexpr int k = decltype(kI)::value;
-    if constexpr (k % 2 == 0) {
-      const V h = p[k / 2];
-      p[k] = mkc<V>(h.x * h.x - h.y * h.y, (h.x + h.x) * h.y);
-    } else {
-      p[k] = cmul(p[k - 1], w);
-    }
-  });
-}
-
 template <int R> struct FirstFactor {
-  static constexpr int v = (R % 4 == 0 && R != 4) ? 4
+  static constexpr int v = R == 30 ? 5                     // 5, 2, 3: the least rounding of its orders
+                         : (R % 4 == 0 && R != 4) ? 4
                          : (R % 2 == 0 && R != 2) ? 2
                          : (R % 3 == 0 && R != 3) ? 3
                          : (R % 5 == 0 && R != 5) ? 5 : R;

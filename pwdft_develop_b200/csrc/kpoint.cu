@@ -110,7 +110,7 @@ int pw_set_kpoint(pw_ctx* ctx, const double k[3]) {
         te[i] = b / (b + 16.0 * a * a * a * a);
       }
   int rc;
-  if ((rc = upload_real(ctx, ctx->ekin_k, ek.data(), nt)) || (rc = upload_real(ctx, ctx->teter_k, te.data(), nt)))
+  if ((rc = upload_spectrum(ctx, ctx->ekin_k, ctx->ekin_k_t, ek.data())) || (rc = upload_real(ctx, ctx->teter_k, te.data(), nt)))
     return rc;
   const int np = (int)ctx->h_pnp.size();
   ctx->qk.release();
@@ -177,12 +177,13 @@ int pw_set_kpoints(pw_ctx* ctx, int nk, const double* kpts) {
   const size_t esz = ctx->esz;
   const int np = (int)ctx->h_pnp.size();
   int rc;
-  if ((rc = ctx->ekin_kb.alloc((size_t)nk * nt * esz))) return rc;
+  if ((rc = ctx->ekin_kb.alloc((size_t)nk * nt * esz)) || (rc = ctx->ekin_kb_t.alloc((size_t)nk * nt * esz))) return rc;
   if (np > 0 && (rc = ctx->qkb.alloc((size_t)nk * np * nt * 2 * esz))) return rc;
   const bool tc = kq_tensor_cores(ctx) && np > 0;
   for (int k = 0; k < nk; ++k) {
     if ((rc = pw_set_kpoint(ctx, kpts + 3 * k))) return rc;
     PWB_CUDA(cudaMemcpy((char*)ctx->ekin_kb.p + (size_t)k * nt * esz, ctx->ekin_k.p, nt * esz, cudaMemcpyDeviceToDevice));
+    PWB_CUDA(cudaMemcpy((char*)ctx->ekin_kb_t.p + (size_t)k * nt * esz, ctx->ekin_k_t.p, nt * esz, cudaMemcpyDeviceToDevice));
     if (np > 0)
       PWB_CUDA(cudaMemcpy((char*)ctx->qkb.p + (size_t)k * np * nt * 2 * esz, ctx->qk.p, (size_t)np * nt * 2 * esz,
                           cudaMemcpyDeviceToDevice));

@@ -32,6 +32,7 @@
 #include "fft.cuh"
 #include "gemm.hpp"
 #include "grid_registry.hpp"
+#include "regfft.cuh"
 
 namespace pwb {
 
@@ -48,7 +49,7 @@ constexpr int PENCIL_THREADS = 256;
 
 template <typename T> using VT = typename C2<T>::t;
 
-// Shared-memory layout of the coarse plane kernels (k_cxy_*, k_exx_*): row y
+// Shared-memory layout of the coarse plane kernels (k_cxy_*): row y
 // at y P0, FR / FC the first-pass lane maps (smem_fft_c's FB) of the x (row)
 // and y (column) transforms.  The specialised planes use the pitch and maps
 // with the fewest shared-memory wavefronts in a bank model of their 8- /
@@ -480,98 +481,6 @@ k_fplane(VT<T>* __restrict__ BC, const T* __restrict__ vtot, NLArgs nl, VT<T>* _
 
 
 // ---------------------------------------------------------------------------
-// exact exchange pair fields (AddMultSpinorEXX, src/SCF/spinor.cpp:682-781).
-// Field f = (band k0 + f / njp, orbital pair jp = f % njp): the plane of
-// psi_k (phi_ja + i phi_jb), ja = j0 + 2 jp, jb = ja + 1 (zero past nphi),
-// forward 2-D FFT in shared memory, stored like k_cxy_fwd's output.
-// ---------------------------------------------------------------------------
-template <typename T, int N0, int N1>
-__global__ void __launch_bounds__(PLANE_THREADS)
-k_exx_fwd(const T* __restrict__ psi, int ld, int k0, const T* __restrict__ phi, int ldp, int j0, int nphi, int njp,
-          VT<T>* __restrict__ A, const VT<T>* twx_g, const VT<T>* twy_g) {
-  using V = VT<T>;
-  using PL = PlaneLayout<T, N0, N1>;
-  constexpr int P0 = PL::P0;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  V* pl = reinterpret_cast<V*>(smraw);
-  V* twx = pl + N1 * P0;
-  V* twy = twx + N0;
-  load_tw(twx, twx_g, N0);
-  load_tw(twy, twy_g, N1);
-  const int z = blockIdx.x, f = blockIdx.y;
-  const int kk = f / njp, jp = f - kk * njp;
-  const long ntot_plane = (long)N0 * N1;
-  const int ja = j0 + 2 * jp, jb = ja + 1;
-  const T* pk = psi + (long)(k0 + kk) * ld + z * ntot_plane;
-  const T* pa = phi + (long)ja * ldp + z * ntot_plane;
-  const T* pb = (jb < nphi) ? phi + (long)jb * ldp + z * ntot_plane : nullptr;
-  for (int i = threadIdx.x; i < N0 * N1; i += blockDim.x) {
-    const int y = i / N0, x = i - y * N0;
-    const T v = pk[i];
-    pl[y * P0 + x] = mkc<V>(v * pa[i], pb ? v * pb[i] : (T)0);
-  }
-  __syncthreads();
-  smem_fft_cb<N0, -1, 1, P0, PL::FR>(pl, N1, twx);
-  __syncthreads();
-  smem_fft_cb<N1, -1, P0, 1, PL::FC>(pl, N0, twy);
-  __syncthreads();
-  const int N2 = gridDim.x;
-  V* Ap = A + ((long)f * N2 + z) * ntot_plane;
-  for (int i = threadIdx.x; i < N0 * N1; i += blockDim.x) {
-    const int y = i / N0, x = i - y * N0;
-    Ap[i] = pl[y * P0 + x];
-  }
-}
-
-// inverse 2-D FFT of the njp fields of band k0 + blockIdx.y on plane z and
-// out_k (+)= sum_jp w_ja phi_ja Re + w_jb phi_jb Im, accumulated in shared memory
-template <typename T, int N0, int N1>
-__global__ void __launch_bounds__(PLANE_THREADS)
-k_exx_inv(const VT<T>* __restrict__ A, int njp, const T* __restrict__ phi, int ldp, int j0, int nphi,
-          const T* __restrict__ wj, T* __restrict__ out, int ldo, int k0, int accumulate, const VT<T>* twx_g,
-          const VT<T>* twy_g) {
-  using V = VT<T>;
-  using PL = PlaneLayout<T, N0, N1>;
-  constexpr int P0 = PL::P0;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  V* pl = reinterpret_cast<V*>(smraw);
-  V* twx = pl + N1 * P0;
-  V* twy = twx + N0;
-  T* acc = reinterpret_cast<T*>(twy + N1);
-  load_tw(twx, twx_g, N0);
-  load_tw(twy, twy_g, N1);
-  const int z = blockIdx.x, kk = blockIdx.y;
-  const int N2 = gridDim.x;
-  const long ntot_plane = (long)N0 * N1;
-  for (int i = threadIdx.x; i < N0 * N1; i += blockDim.x) acc[i] = (T)0;
-  for (int jp = 0; jp < njp; ++jp) {
-    const V* Dp = A + ((long)(kk * njp + jp) * N2 + z) * ntot_plane;
-    __syncthreads();
-    for (int i = threadIdx.x; i < N0 * N1; i += blockDim.x) {
-      const int y = i / N0, x = i - y * N0;
-      pl[y * P0 + x] = Dp[i];
-    }
-    __syncthreads();
-    smem_fft_cb<N1, +1, P0, 1, PL::FC>(pl, N0, twy);
-    __syncthreads();
-    smem_fft_cb<N0, +1, 1, P0, PL::FR>(pl, N1, twx);
-    __syncthreads();
-    const int ja = j0 + 2 * jp, jb = ja + 1;
-    const T wa = wj[ja], wb = (jb < nphi) ? wj[jb] : (T)0;
-    const T* pa = phi + (long)ja * ldp + z * ntot_plane;
-    const T* pb = (jb < nphi) ? phi + (long)jb * ldp + z * ntot_plane : pa;
-    for (int i = threadIdx.x; i < N0 * N1; i += blockDim.x) {
-      const int y = i / N0, x = i - y * N0;
-      const V v = pl[y * P0 + x];
-      acc[i] += wa * pa[i] * v.x + wb * pb[i] * v.y;
-    }
-  }
-  __syncthreads();
-  T* o = out + (long)(k0 + kk) * ldo + z * ntot_plane;
-  for (int i = threadIdx.x; i < N0 * N1; i += blockDim.x) o[i] = accumulate ? o[i] + acc[i] : acc[i];
-}
-
-// ---------------------------------------------------------------------------
 // fine plane, local potential only (the projectors are applied on the coarse
 // grid as dense GEMMs): IFFT y on the slot columns, then per warp a group of
 // rows: IFFT x, * V_loc, FFT x, truncate; FFT y; truncate.  MODE 1 starts
@@ -722,53 +631,17 @@ template <int NXF> struct FlocLayoutPlain {
 template <typename T, int NXF, int NYF, int VAR>
 using FlocLayoutVar = typename std::conditional<VAR == 1, FlocLayoutPlain<NXF>, FlocLayout<T, NXF, NYF>>::type;
 
-// Lane order of the local potential for the row pass of k_floc2 (fft_variant
-// 2): lane f NX1 + k1 of a warp holds row r0 + f (rows in groups of FX) and
-// needs V(x = k1 + NX1 k2) for k2 = 0 .. NX2-1.  The permuted copy stores, per
-// fine plane and row group, NQ blocks of 32 lanes x VW consecutive k2 values,
-// so each vector load of a warp reads 32 VW contiguous reals.  Unused lanes
-// (rows past the plane, lanes past FX NX1) hold zeros.
-template <typename T, int NXF, int NYF> struct VpermLayout {
-  static constexpr int NX1 = Split<NXF>::n1, NX2 = NXF / NX1, FX = 32 / NX1;
-  static constexpr int VW = 16 / (int)sizeof(T);                // reals per 16-byte load
-  static constexpr bool OK = NX2 % VW == 0;
-  static constexpr int NQ = NX2 / VW, NG = (NYF + FX - 1) / FX;
-  static constexpr long PLANE = (long)NG * NQ * 32 * VW;        // reals per fine plane
-};
-template <typename T, int NXF, int NYF>
-__global__ void k_vperm(const T* __restrict__ v, T* __restrict__ vp, int nzf) {
-  using LY = VpermLayout<T, NXF, NYF>;
-  const long total = LY::PLANE * nzf;
-  for (long o = blockIdx.x * (long)blockDim.x + threadIdx.x; o < total; o += (long)gridDim.x * blockDim.x) {
-    const long zf = o / LY::PLANE;
-    long r = o - zf * LY::PLANE;
-    const int i = (int)(r % LY::VW);
-    r /= LY::VW;
-    const int lane = (int)(r % 32);
-    r /= 32;
-    const int q = (int)(r % LY::NQ);
-    const int g = (int)(r / LY::NQ);
-    const int f = lane / LY::NX1, k1 = lane - f * LY::NX1;
-    const int y = g * LY::FX + f, x = k1 + LY::NX1 * (q * LY::VW + i);
-    vp[o] = (f < LY::FX && y < NYF) ? v[(zf * NYF + y) * NXF + x] : (T)0;
-  }
-}
-
 // VAR selects the radix decomposition of the x and y transforms (0: Split,
-// 1: SplitAlt) and where the inter-stage twiddles come from (0, 1: the shared
-// tables; 2: Split with W^{j k} formed in registers from one table entry per
-// transform), the autotuner's FFT candidates
+// 1: SplitAlt), the autotuner's candidates beside the register transforms
 template <typename T, int NXF, int NYF, int VAR = 0>
 __global__ void __launch_bounds__(FLOC_THREADS, sizeof(T) == 4 ? 3 : 1)
-k_floc2(VT<T>* __restrict__ BC, const T* __restrict__ vtot, T inv_nf, const VT<T>* twx_g, const VT<T>* twy_g,
-        const T* __restrict__ vperm) {
+k_floc2(VT<T>* __restrict__ BC, const T* __restrict__ vtot, T inv_nf, const VT<T>* twx_g, const VT<T>* twy_g) {
   using V = VT<T>;
   constexpr int n0 = NXF / 2;
   constexpr int nsx = n0 + 1, nsy = NYF / 2 + 1;
   using LY = FlocLayoutVar<T, NXF, NYF, VAR>;
   constexpr int PS = LY::PS, SKS = LY::SKS, PR = LY::PR, SKR = LY::SKR;
   constexpr bool FA = LY::FA, FB = LY::FB;
-  constexpr bool RTW = VAR == 2;
   constexpr int NX1 = SplitVar<NXF, VAR>::n1, NX2 = NXF / NX1, FX = 32 / NX1;
   constexpr int NY1 = SplitVar<NYF, VAR>::n1, NY2 = NYF / NY1, FY = 32 / NY1;
   constexpr int RX = (FX * NX2 + 31) / 32;
@@ -787,10 +660,7 @@ k_floc2(VT<T>* __restrict__ BC, const T* __restrict__ vtot, T inv_nf, const VT<T
   __syncthreads();
 
   // A: inverse y transform of the nsx slot columns, GA columns per warp step
-  // (variant 2: twice the FY of the second pass when that fills whole warp
-  // rounds in the first pass, 96: 8 columns x 12 = 3 rounds instead of 4 x 12
-  // in two half-empty rounds)
-  constexpr int GA = (RTW && (2 * FY * NY2) % 32 == 0) ? 2 * FY : FY;
+  constexpr int GA = FY;
   constexpr int RA = (GA * NY2 + 31) / 32;
   for (int g = warp * GA; g < nsx; g += nw * GA) {
 #pragma unroll
@@ -802,29 +672,15 @@ k_floc2(VT<T>* __restrict__ BC, const T* __restrict__ vtot, T inv_nf, const VT<T
         V t[NY1];
         sfor<0, NY1>([&](auto jI) {
           constexpr int j1 = decltype(jI)::value;
-          if constexpr (!RTW || any_slot<NYF>(NY2 * j1, NY2)) {
-            const int s = fine_slot<NYF>(NY2 * j1 + j2);
-            t[j1] = s >= 0 ? Bp[s * nsx + c] : mkc<V>(0, 0);
-          } else {
-            t[j1] = mkc<V>(0, 0);
-          }
+          const int s = fine_slot<NYF>(NY2 * j1 + j2);
+          t[j1] = s >= 0 ? Bp[s * nsx + c] : mkc<V>(0, 0);
         });
-        if constexpr (RTW) DFTZ<NY1, +1, V, zero_inputs<NYF, NY1, NY2>()>::run(t);
-        else DFT<NY1, +1, V>::run(t);
-        if constexpr (RTW) {
-          V p_[NY1];
-          V w = twy[j2];
+        DFT<NY1, +1, V>::run(t);
+#pragma unroll
+        for (int k1 = 1; k1 < NY1; ++k1) {
+          V w = twy[j2 * k1];
           w.y = -w.y;
-          twiddle_powers<NY1>(w, p_);
-#pragma unroll
-          for (int k1 = 1; k1 < NY1; ++k1) t[k1] = cmul(t[k1], p_[k1]);
-        } else {
-#pragma unroll
-          for (int k1 = 1; k1 < NY1; ++k1) {
-            V w = twy[j2 * k1];
-            w.y = -w.y;
-            t[k1] = cmul(t[k1], w);
-          }
+          t[k1] = cmul(t[k1], w);
         }
 #pragma unroll
         for (int k1 = 0; k1 < NY1; ++k1) S[(NY2 * k1 + j2) * PS + SKS * k1 + c] = t[k1];
@@ -868,29 +724,15 @@ k_floc2(VT<T>* __restrict__ BC, const T* __restrict__ vtot, T inv_nf, const VT<T
         const V* srow = S + (r0 + f) * PS + SKS * ((r0 + f) / NY2);
         sfor<0, NX1>([&](auto jI) {
           constexpr int j1 = decltype(jI)::value;
-          if constexpr (!RTW || any_slot<NXF>(NX2 * j1, NX2)) {
-            const int s = fine_slot<NXF>(NX2 * j1 + j2);
-            t[j1] = s >= 0 ? srow[s] : mkc<V>(0, 0);
-          } else {
-            t[j1] = mkc<V>(0, 0);
-          }
+          const int s = fine_slot<NXF>(NX2 * j1 + j2);
+          t[j1] = s >= 0 ? srow[s] : mkc<V>(0, 0);
         });
-        if constexpr (RTW) DFTZ<NX1, +1, V, zero_inputs<NXF, NX1, NX2>()>::run(t);
-        else DFT<NX1, +1, V>::run(t);
-        if constexpr (RTW) {
-          V p_[NX1];
-          V w = twx[j2];
+        DFT<NX1, +1, V>::run(t);
+#pragma unroll
+        for (int k1 = 1; k1 < NX1; ++k1) {
+          V w = twx[j2 * k1];
           w.y = -w.y;
-          twiddle_powers<NX1>(w, p_);
-#pragma unroll
-          for (int k1 = 1; k1 < NX1; ++k1) t[k1] = cmul(t[k1], p_[k1]);
-        } else {
-#pragma unroll
-          for (int k1 = 1; k1 < NX1; ++k1) {
-            V w = twx[j2 * k1];
-            w.y = -w.y;
-            t[k1] = cmul(t[k1], w);
-          }
+          t[k1] = cmul(t[k1], w);
         }
 #pragma unroll
         for (int k1 = 0; k1 < NX1; ++k1) Rw[f * PR + (NX2 + SKR) * k1 + j2] = t[k1];
@@ -906,38 +748,12 @@ k_floc2(VT<T>* __restrict__ BC, const T* __restrict__ vtot, T inv_nf, const VT<T
 #pragma unroll
         for (int j2 = 0; j2 < NX2; ++j2) u[j2] = rr[j2];
         DFT<NX2, +1, V>::run(u);                    // u[k2] = x[k1 + NX1 k2]
-        if constexpr (RTW && VpermLayout<T, NXF, NYF>::OK) {
-          using PL = VpermLayout<T, NXF, NYF>;
-          using VV = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-          const VV* vq = reinterpret_cast<const VV*>(vperm + ((long)zf * PL::NG + r0 / FX) * PL::NQ * 32 * PL::VW) + lane;
+        const T* vrow = vtot + ((long)zf * NYF + r0 + f) * NXF + k1;
 #pragma unroll
-          for (int q = 0; q < PL::NQ; ++q) {
-            const VV vv = vq[32 * q];
-            if constexpr (sizeof(T) == 4) {
-              u[4 * q + 0] = cscale(u[4 * q + 0], (T)vv.x);
-              u[4 * q + 1] = cscale(u[4 * q + 1], (T)vv.y);
-              u[4 * q + 2] = cscale(u[4 * q + 2], (T)vv.z);
-              u[4 * q + 3] = cscale(u[4 * q + 3], (T)vv.w);
-            } else {
-              u[2 * q + 0] = cscale(u[2 * q + 0], (T)vv.x);
-              u[2 * q + 1] = cscale(u[2 * q + 1], (T)vv.y);
-            }
-          }
-        } else {
-          const T* vrow = vtot + ((long)zf * NYF + r0 + f) * NXF + k1;
-#pragma unroll
-          for (int k2 = 0; k2 < NX2; ++k2) u[k2] = cscale(u[k2], vrow[NX1 * k2]);
-        }
+        for (int k2 = 0; k2 < NX2; ++k2) u[k2] = cscale(u[k2], vrow[NX1 * k2]);
         DFT<NX2, -1, V>::run(u);                    // forward, first stage over k2
-        if constexpr (RTW) {
-          V p_[NX2];
-          twiddle_powers<NX2>(twx[k1], p_);
 #pragma unroll
-          for (int m2 = 1; m2 < NX2; ++m2) u[m2] = cmul(u[m2], p_[m2]);
-        } else {
-#pragma unroll
-          for (int m2 = 1; m2 < NX2; ++m2) u[m2] = cmul(u[m2], twx[k1 * m2]);
-        }
+        for (int m2 = 1; m2 < NX2; ++m2) u[m2] = cmul(u[m2], twx[k1 * m2]);
 #pragma unroll
         for (int m2 = 0; m2 < NX2; ++m2) rr[m2] = u[m2];
       }
@@ -955,10 +771,8 @@ k_floc2(VT<T>* __restrict__ BC, const T* __restrict__ vtot, T inv_nf, const VT<T
         V* srow = S + (r0 + f) * PS + SKS * ((r0 + f) / NY2);
         sfor<0, NX1>([&](auto mI) {
           constexpr int m1 = decltype(mI)::value;
-          if constexpr (!RTW || any_slot<NXF>(NX2 * m1, NX2)) {
-            const int s = fine_slot<NXF>(m2 + NX2 * m1);
-            if (s >= 0) srow[s] = t[m1];
-          }
+          const int s = fine_slot<NXF>(m2 + NX2 * m1);
+          if (s >= 0) srow[s] = t[m1];
         });
       }
     }
@@ -978,15 +792,8 @@ k_floc2(VT<T>* __restrict__ BC, const T* __restrict__ vtot, T inv_nf, const VT<T
 #pragma unroll
         for (int j1 = 0; j1 < NY1; ++j1) t[j1] = S[(NY2 * j1 + j2) * PS + SKS * j1 + c];
         DFT<NY1, -1, V>::run(t);
-        if constexpr (RTW) {
-          V p_[NY1];
-          twiddle_powers<NY1>(twy[j2], p_);
 #pragma unroll
-          for (int k1 = 1; k1 < NY1; ++k1) t[k1] = cmul(t[k1], p_[k1]);
-        } else {
-#pragma unroll
-          for (int k1 = 1; k1 < NY1; ++k1) t[k1] = cmul(t[k1], twy[j2 * k1]);
-        }
+        for (int k1 = 1; k1 < NY1; ++k1) t[k1] = cmul(t[k1], twy[j2 * k1]);
 #pragma unroll
         for (int k1 = 0; k1 < NY1; ++k1) S[(NY2 * k1 + j2) * PS + SKS * k1 + c] = t[k1];
       }
@@ -1003,10 +810,8 @@ k_floc2(VT<T>* __restrict__ BC, const T* __restrict__ vtot, T inv_nf, const VT<T
         DFT<NY2, -1, V>::run(u);
         sfor<0, NY2>([&](auto kI) {
           constexpr int k2 = decltype(kI)::value;
-          if constexpr (!RTW || any_slot<NYF>(NY1 * k2, NY1)) {
-            const int s = fine_slot<NYF>(k1 + NY1 * k2);
-            if (s >= 0) Bp[s * nsx + c] = cscale(u[k2], inv_nf);
-          }
+          const int s = fine_slot<NYF>(k1 + NY1 * k2);
+          if (s >= 0) Bp[s * nsx + c] = cscale(u[k2], inv_nf);
         });
       }
     }
@@ -1275,40 +1080,6 @@ k_zfold(const VT<T>* __restrict__ C, const VT<T>* __restrict__ K, VT<T>* __restr
   }
 }
 
-// z pencils for the Teter preconditioner: FFT z, * teter / N_c, IFFT z
-template <typename T, int NZ, int TX>
-__global__ void __launch_bounds__(PENCIL_THREADS, sizeof(T) == 4 ? 4 : 1)
-k_zteter(VT<T>* __restrict__ A, const T* __restrict__ teter, int n0, int n1, T inv_nc, const VT<T>* twz_g) {
-  using V = VT<T>;
-  constexpr int PI = TX + 1;
-  extern __shared__ __align__(16) unsigned char smraw[];
-  V* in = reinterpret_cast<V*>(smraw);
-  V* twz = in + NZ * PI;
-  load_tw(twz, twz_g, NZ);
-  const int ky = blockIdx.x, kx0 = blockIdx.y * TX, p = blockIdx.z;
-  const int tw = min(TX, n0 - kx0);
-  const long nplane = (long)n0 * n1;
-  V* Ap = A + (long)p * NZ * nplane;
-  for (int i = threadIdx.x; i < NZ * TX; i += blockDim.x) {
-    const int z = i / TX, c = i - z * TX;
-    in[z * PI + c] = (c < tw) ? Ap[z * nplane + (long)ky * n0 + kx0 + c] : mkc<V>(0, 0);
-  }
-  __syncthreads();
-  smem_fft_cb<NZ, -1, PI, 1>(in, tw, twz);
-  __syncthreads();
-  for (int i = threadIdx.x; i < NZ * TX; i += blockDim.x) {
-    const int kz = i / TX, c = i - kz * TX;
-    if (c < tw) in[kz * PI + c] = cscale(in[kz * PI + c], teter[kz * nplane + (long)ky * n0 + kx0 + c] * inv_nc);
-  }
-  __syncthreads();
-  smem_fft_cb<NZ, +1, PI, 1>(in, tw, twz);
-  __syncthreads();
-  for (int i = threadIdx.x; i < NZ * TX; i += blockDim.x) {
-    const int z = i / TX, c = i - z * TX;
-    if (c < tw) Ap[z * nplane + (long)ky * n0 + kx0 + c] = in[z * PI + c];
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Sphere-cut (G-space) mode, Spinor::AddMultSpinorFineR2C complex overload
 // (src/SCF/spinor.cpp:528-680).  A band is its coefficients c_s on the half
@@ -1492,6 +1263,10 @@ k_cxy_inv(const VT<T>* __restrict__ D, T* __restrict__ out, int ldo, int nband, 
   }
 }
 
+}  // namespace pwb
+#include "pipeline_reg.cuh"
+namespace pwb {
+
 // ---------------------------------------------------------------------------
 // host-side launch plan for one (precision, grid) instantiation
 // ---------------------------------------------------------------------------
@@ -1516,14 +1291,73 @@ struct Plan {
   static constexpr int TXF = TX;   // z-fold tile width
   using V = VT<T>;
   static constexpr int NF0 = 2 * N0, NF1 = 2 * N1, NF2 = 2 * N2;
+  // register-resident transforms along every axis (pipeline_reg.cuh): Teter and
+  // exchange always, H*psi in fft_variant 2 (the autotuner's other candidates
+  // keep the shared-memory kernels)
+  static_assert(RegN<T, N0>::OK && RegN<T, N1>::OK && RegN<T, N2>::OK, "grid length without a register transform");
+  static bool reg(const pw_ctx* c) { return c->fft_variant == 2; }
+  using RP = RPlane<T, N0, N1>;
+  using RZ = RPencil<T, N2>;
+  static dim3 rplane_grid(int fields) { return dim3((N2 + RP::NPL - 1) / RP::NPL, fields); }
+  static dim3 rzp_grid(int fields) { return dim3((N0 * N1 + RZ::COLSP - 1) / RZ::COLSP, fields); }
+  static dim3 rz_grid(int fields) { return dim3((N0 * N1 + RZ::COLS - 1) / RZ::COLS, fields); }
+  static size_t sm_rexx_inv() { return RP::smem + sizeof(T) * RegN<T, N1>::M * RP::TH; }
+
+  static int set_attrs_reg() {
+    static PerDeviceOnce once;
+    if (once.done()) return PW_OK;
+    auto big = [](const void* f, size_t n) {
+      return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)n);
+    };
+    PWB_CUDA(big((const void*)k_rfwd<T, N0, N1, 0>, RP::smem));
+    PWB_CUDA(big((const void*)k_rfwd<T, N0, N1, 1>, RP::smem));
+    PWB_CUDA(big((const void*)k_rfwd<T, N0, N1, 2>, RP::smem));
+    PWB_CUDA(big((const void*)k_rinv<T, N0, N1, false>, RP::smem));
+    PWB_CUDA(big((const void*)k_rinv<T, N0, N1, true>, RP::smem));
+    PWB_CUDA(big((const void*)k_rexx_inv<T, N0, N1>, sm_rexx_inv()));
+    PWB_CUDA(big((const void*)k_rfloc<T, N0, N1>, RFine<T, N0, N1>::smem));
+    PWB_CUDA(big((const void*)k_rfloc<T, N1, N0>, RFine<T, N1, N0>::smem));
+    once.mark();
+    return PW_OK;
+  }
+
+  // psi -> slot field BC and kinetic spectrum K (reg form); fwd 0: band pairs, 1: complex bands
+  template <int MODE>
+  static void reg_up(pw_ctx* c, const T* psi, int ld, int nband, int band0, int fields, const T* ekin, int kf0, int fpk,
+                     long kstride, cudaStream_t st) {
+    V* AD = reinterpret_cast<V*>(c->s_ad.p);
+    { Launch L_(c, st, KK_CXY_FWD);
+    k_rfwd<T, N0, N1, MODE><<<rplane_grid(fields), RP::TH, RP::smem, st>>>(psi, ld, nband, band0, nullptr, RExx{}, AD,
+                                                                         N2); }
+    { Launch L_(c, st, KK_ZPAD);
+    k_rzpad<T, N0, N1, N2><<<rzp_grid(fields), RZ::THP, 0, st>>>(
+        AD, reinterpret_cast<V*>(c->s_k.p), reinterpret_cast<V*>(c->s_bc.p), ekin, (T)(1.0 / (double)c->ntot),
+        tw(c, 5), MODE, kf0, fpk, kstride); }
+  }
+  // local potential on the slot field, fold to the coarse [z][kx][ky] field
+  static void reg_down(pw_ctx* c, int fields, int cplx, const T* mask, cudaStream_t st) {
+    V* BC = reinterpret_cast<V*>(c->s_bc.p);
+    V* AD = reinterpret_cast<V*>(c->s_ad.p);
+    const V* K = reinterpret_cast<const V*>(c->s_k.p);
+    { Launch L_(c, st, KK_FPLANE_APPLY);
+    k_rfloc<T, N0, N1><<<dim3(NF2, fields), RFine<T, N0, N1>::TH, RFine<T, N0, N1>::smem, st>>>(
+        BC, reinterpret_cast<const T*>(c->vtot.p), (T)(1.0 / (double)c->ntotf), tw(c, 3), tw(c, 4)); }
+    Launch L_(c, st, KK_ZFOLD);
+    if (mask) k_rzfold<T, N0, N1, N2, true><<<rz_grid(fields), RZ::TH, 0, st>>>(BC, K, AD, tw(c, 5), cplx, mask);
+    else k_rzfold<T, N0, N1, N2, false><<<rz_grid(fields), RZ::TH, 0, st>>>(BC, K, AD, tw(c, 5), cplx, nullptr);
+  }
+  template <bool CPLX>
+  static void reg_out(pw_ctx* c, T* out, int ldo, int nband, int band0, int fields, int accumulate, cudaStream_t st) {
+    Launch L_(c, st, KK_CXY_INV);
+    k_rinv<T, N0, N1, CPLX><<<rplane_grid(fields), RP::TH, RP::smem, st>>>(reinterpret_cast<const V*>(c->s_ad.p), out,
+                                                                          ldo, nband, band0, accumulate, N2);
+  }
 
   static int chunk_rows() { return fplane_cr<T>(NF0, NF1); }
 
   static size_t sm_cxy() { return sizeof(V) * (N1 * PlaneLayout<T, N0, N1>::P0 + N0 + N1); }
   static size_t sm_zpad() { return sizeof(V) * (N2 * (TX + 1) + NF2 * (2 * TX + 1) + N2 + NF2); }
   static size_t sm_zfold() { return sizeof(V) * (NF2 * (2 * TXF + 1) + N2 * (TXF + 1) + N2 + NF2); }
-  static size_t sm_zteter() { return sizeof(V) * (N2 * (TX + 1) + N2); }
-  static size_t sm_exx_inv() { return sm_cxy() + sizeof(T) * N0 * N1; }
   static size_t sm_floc() {
     return sizeof(V) * ((size_t)NF1 * (N0 + 1) + NF0 + NF1 + (size_t)(FLOC_THREADS / 32) * FftGroup<NF0>::f * (NF0 + 1));
   }
@@ -1532,29 +1366,16 @@ struct Plan {
     return sizeof(V) * ((size_t)floc_s_size<LY, NF1, NF1 / SplitVar<NF1, VAR>::n1>() + NF0 + NF1 +
                         (size_t)(FLOC_THREADS / 32) * (32 / SplitVar<NF0, VAR>::n1) * LY::PR);
   }
-  // the fused fine-plane kernel in the context's radix decomposition
+  // the fused fine-plane kernel in the context's form
   static void launch_floc2(pw_ctx* c, V* BC, const T* vt, T inv_nf, int nblk, cudaStream_t st) {
-    const T* vp = reinterpret_cast<const T*>(c->vperm.p);
-    if (c->fft_variant == 2 && (vp || !VpermLayout<T, NF0, NF1>::OK))
-      k_floc2<T, NF0, NF1, 2><<<dim3(NF2, nblk), FLOC_THREADS, sm_floc2<2>(), st>>>(BC, vt, inv_nf, tw(c, 3), tw(c, 4),
-                                                                                   vp);
+    if (c->fft_variant == 2 && c->gs)
+      // sphere-cut slots are [ky][kx]: the axes and the potential change places
+      k_rfloc<T, N1, N0><<<dim3(NF2, nblk), RFine<T, N1, N0>::TH, RFine<T, N1, N0>::smem, st>>>(
+          BC, reinterpret_cast<const T*>(c->vtot_t.p), inv_nf, tw(c, 4), tw(c, 3));
     else if (c->fft_variant == 1)
-      k_floc2<T, NF0, NF1, 1><<<dim3(NF2, nblk), FLOC_THREADS, sm_floc2<1>(), st>>>(BC, vt, inv_nf, tw(c, 3), tw(c, 4),
-                                                                                   nullptr);
+      k_floc2<T, NF0, NF1, 1><<<dim3(NF2, nblk), FLOC_THREADS, sm_floc2<1>(), st>>>(BC, vt, inv_nf, tw(c, 3), tw(c, 4));
     else
-      k_floc2<T, NF0, NF1, 0><<<dim3(NF2, nblk), FLOC_THREADS, sm_floc2<0>(), st>>>(BC, vt, inv_nf, tw(c, 3), tw(c, 4),
-                                                                                   nullptr);
-  }
-  // pw_ctx::vperm from pw_ctx::vtot (the lane order of VpermLayout)
-  static int vperm_build(pw_ctx* c, cudaStream_t st) {
-    using PL = VpermLayout<T, NF0, NF1>;
-    if (!PL::OK || !c->vtot.p) return PW_OK;
-    int rc = c->vperm.alloc((size_t)PL::PLANE * NF2 * sizeof(T));
-    if (rc) return rc;
-    k_vperm<T, NF0, NF1><<<148 * 4, 256, 0, st>>>(reinterpret_cast<const T*>(c->vtot.p),
-                                                   reinterpret_cast<T*>(c->vperm.p), NF2);
-    PWB_CUDA(cudaGetLastError());
-    return PW_OK;
+      k_floc2<T, NF0, NF1, 0><<<dim3(NF2, nblk), FLOC_THREADS, sm_floc2<0>(), st>>>(BC, vt, inv_nf, tw(c, 3), tw(c, 4));
   }
   static size_t sm_fplane(int cr) {
     return sizeof(V) * ((size_t)NF1 * (N0 + 1) + (size_t)cr * (NF0 + 1) + NF0 + NF1);
@@ -1570,12 +1391,12 @@ struct Plan {
     PWB_CUDA(cudaFuncSetAttribute(k_zfold<T, N2, NF2, TXF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_zfold()));
     PWB_CUDA(cudaFuncSetAttribute(k_cxy_fwd<T, N0, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_cxy()));
     PWB_CUDA(cudaFuncSetAttribute(k_cxy_inv<T, N0, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_cxy()));
-    PWB_CUDA(cudaFuncSetAttribute(k_zteter<T, N2, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_zteter()));
     PWB_CUDA(cudaFuncSetAttribute(k_floc<T, NF0, NF1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_floc()));
     PWB_CUDA(cudaFuncSetAttribute(k_floc2<T, NF0, NF1, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_floc2<0>()));
     PWB_CUDA(cudaFuncSetAttribute(k_floc2<T, NF0, NF1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_floc2<1>()));
-    PWB_CUDA(cudaFuncSetAttribute(k_floc2<T, NF0, NF1, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_floc2<2>()));
     PWB_CUDA(cudaFuncSetAttribute(k_floc<T, NF0, NF1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_floc()));
+    int rc = set_attrs_reg();
+    if (rc) return rc;
     once.mark();
     return PW_OK;
   }
@@ -1617,6 +1438,17 @@ struct Plan {
         return rc;
       }
       PWB_CUDA(cudaEventRecord(c->nl_join, sn));
+    }
+    if (reg(c) && c->nl_mode == PW_NL_DENSE) {
+      reg_up<0>(c, psi, ld, nband, band0, npair, reinterpret_cast<const T*>(c->ekin_t.p), 0, 1 << 30, 0, st);
+      reg_down(c, npair, 0, filt ? reinterpret_cast<const T*>(c->wmask_t.p) : nullptr, st);
+      if (sn) PWB_CUDA(cudaStreamWaitEvent(st, c->nl_join, 0));
+      reg_out<false>(c, out, ldo, nband, band0, npair, sn ? 1 : accumulate, st);
+      PWB_CUDA(cudaGetLastError());
+      if (dense_nl && !sn)
+        if ((rc = dense_apply(c, nl_set(c, filt), psi + (long)band0 * ld, ld, out + (long)band0 * ldo, ldo, nbnl, st)))
+          return rc;
+      return exchange_batch(c, psi, ld, out, ldo, nband, band0, npair, st, filt);
     }
     { Launch L_(c, st, KK_CXY_FWD);
     k_cxy_fwd<T, N0, N1><<<dim3(N2, npair), PLANE_THREADS, sm_cxy(), st>>>(psi, ld, nband, band0, AD, tw(c, 0), tw(c, 1)); }
@@ -1717,12 +1549,6 @@ struct Plan {
   static int exx_apply(pw_ctx* c, const T* psi, int ld, int nb, T* out, int ldo, int accumulate, cudaStream_t st) {
     int rc = set_attrs();
     if (rc) return rc;
-    static PerDeviceOnce attr;
-    if (!attr.done()) {
-      PWB_CUDA(cudaFuncSetAttribute(k_exx_fwd<T, N0, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_cxy()));
-      PWB_CUDA(cudaFuncSetAttribute(k_exx_inv<T, N0, N1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_exx_inv()));
-      attr.mark();
-    }
     const int nphi = c->exx_nphi;
     if (nphi == 0 || nb == 0) {
       if (!accumulate && nb > 0)
@@ -1738,22 +1564,20 @@ struct Plan {
     V* A = reinterpret_cast<V*>(c->s_exx.p);
     const T* phi = reinterpret_cast<const T*>(c->exx_phi.p);
     const T* wj = reinterpret_cast<const T*>(c->exx_w.p);
-    const T* kern = reinterpret_cast<const T*>(c->exx_kern.p);
+    const T* kern = reinterpret_cast<const T*>(c->exx_kern_t.p);
     const T inv_nc = (T)(1.0 / (double)nt);
-    const int ntx = (N0 + TX - 1) / TX;
     for (int k0 = 0; k0 < nb; k0 += kc) {
       const int nk = std::min(kc, nb - k0);
       for (int jp0 = 0; jp0 < njp; jp0 += jc) {
         const int nj = std::min(jc, njp - jp0);
+        const RExx ex{k0, (int)nt, 2 * jp0, nphi, nj};
         { Launch L_(c, st, KK_EXX);
-        k_exx_fwd<T, N0, N1><<<dim3(N2, nk * nj), PLANE_THREADS, sm_cxy(), st>>>(
-            psi, ld, k0, phi, (int)nt, 2 * jp0, nphi, nj, A, tw(c, 0), tw(c, 1)); }
+        k_rfwd<T, N0, N1, 2><<<rplane_grid(nk * nj), RP::TH, RP::smem, st>>>(psi, ld, 0, 0, phi, ex, A, N2); }
         { Launch L_(c, st, KK_EXX);
-        k_zteter<T, N2, TX><<<dim3(N1, ntx, nk * nj), PENCIL_THREADS, sm_zteter(), st>>>(A, kern, N0, N1, inv_nc, tw(c, 2)); }
+        k_rzmul<T, N0, N1, N2><<<rz_grid(nk * nj), RZ::TH, 0, st>>>(A, kern, inv_nc); }
         { Launch L_(c, st, KK_EXX);
-        k_exx_inv<T, N0, N1><<<dim3(N2, nk), PLANE_THREADS, sm_exx_inv(), st>>>(
-            A, nj, phi, (int)nt, 2 * jp0, nphi, wj, out, ldo, k0, (accumulate || jp0 > 0) ? 1 : 0, tw(c, 0),
-            tw(c, 1)); }
+        k_rexx_inv<T, N0, N1><<<rplane_grid(nk), RP::TH, sm_rexx_inv(), st>>>(
+            A, phi, ex, wj, out, ldo, (accumulate || jp0 > 0) ? 1 : 0, N2); }
         PWB_CUDA(cudaGetLastError());
       }
     }
@@ -1871,6 +1695,12 @@ struct Plan {
     const T inv_nf = (T)(1.0 / (double)c->ntotf);
     const int ntx = (N0 + TX - 1) / TX;
     const T* pr = reinterpret_cast<const T*>(psi);
+    if (reg(c)) {
+      const T* ek = reinterpret_cast<const T*>(ekin_all ? c->ekin_kb_t.p : c->ekin_k_t.p);
+      reg_up<1>(c, pr, ld, 0, band0, nb, ek, band0, fpk, ekin_all ? c->ntot : 0, st);
+      reg_down(c, nb, 1, nullptr, st);
+      reg_out<true>(c, reinterpret_cast<T*>(out), ldo, 0, band0, nb, accumulate, st);
+    } else {
     { Launch L_(c, st, KK_CXY_FWD);
     k_cxy_fwd<T, N0, N1, true><<<dim3(N2, nb), PLANE_THREADS, sm_cxy(), st>>>(pr, ld, 0, band0, AD, tw(c, 0), tw(c, 1)); }
     { Launch L_(c, st, KK_ZPAD);
@@ -1885,6 +1715,7 @@ struct Plan {
     { Launch L_(c, st, KK_CXY_INV);
     k_cxy_inv<T, N0, N1, true><<<dim3(N2, nb), PLANE_THREADS, sm_cxy(), st>>>(AD, reinterpret_cast<T*>(out), ldo, 0,
                                                                               band0, accumulate, tw(c, 0), tw(c, 1)); }
+    }
     PWB_CUDA(cudaGetLastError());
     if (c->nproj == 0 || !(qk_all ? qk_all : c->qk.p)) return PW_OK;
     // V_nl psi = Q diag(d) Q^H psi with the complex coarse projector matrix Q of
@@ -2042,14 +1873,12 @@ struct Plan {
     if (rc) return rc;
     V* AD = reinterpret_cast<V*>(c->s_ad.p);
     const T inv_nc = (T)(1.0 / (double)c->ntot);
-    const int ntx = (N0 + TX - 1) / TX;
     { Launch L_(c, st, KK_CXY_FWD);
-    k_cxy_fwd<T, N0, N1><<<dim3(N2, npair), PLANE_THREADS, sm_cxy(), st>>>(r, ld, nband, band0, AD, tw(c, 0), tw(c, 1)); }
+    k_rfwd<T, N0, N1, 0><<<rplane_grid(npair), RP::TH, RP::smem, st>>>(r, ld, nband, band0, nullptr, RExx{}, AD, N2); }
     { Launch L_(c, st, KK_ZTETER);
-    k_zteter<T, N2, TX><<<dim3(N1, ntx, npair), PENCIL_THREADS, sm_zteter(), st>>>(
-        AD, reinterpret_cast<const T*>(c->teter_tab ? c->teter_tab : c->teter.p), N0, N1, inv_nc, tw(c, 2)); }
-    { Launch L_(c, st, KK_CXY_INV);
-    k_cxy_inv<T, N0, N1><<<dim3(N2, npair), PLANE_THREADS, sm_cxy(), st>>>(AD, out, ldo, nband, band0, accumulate, tw(c, 0), tw(c, 1)); }
+    k_rzmul<T, N0, N1, N2><<<rz_grid(npair), RZ::TH, 0, st>>>(
+        AD, reinterpret_cast<const T*>(c->teter_tab ? c->wmask_t.p : c->teter_t.p), inv_nc); }
+    reg_out<false>(c, out, ldo, nband, band0, npair, accumulate, st);
     PWB_CUDA(cudaGetLastError());
     return PW_OK;
   }
@@ -2062,13 +1891,10 @@ struct Plan {
     if (rc) return rc;
     V* AD = reinterpret_cast<V*>(scratch);
     const T inv_nc = (T)(1.0 / (double)c->ntot);
-    const int ntx = (N0 + TX - 1) / TX;
     c->launches += 3;
-    k_cxy_fwd<T, N0, N1><<<dim3(N2, npair), PLANE_THREADS, sm_cxy(), st>>>(r, ld, nband, band0, AD, tw(c, 0), tw(c, 1));
-    k_zteter<T, N2, TX><<<dim3(N1, ntx, npair), PENCIL_THREADS, sm_zteter(), st>>>(
-        AD, reinterpret_cast<const T*>(c->teter.p), N0, N1, inv_nc, tw(c, 2));
-    k_cxy_inv<T, N0, N1><<<dim3(N2, npair), PLANE_THREADS, sm_cxy(), st>>>(AD, out, ldo, nband, band0, accumulate,
-                                                                            tw(c, 0), tw(c, 1));
+    k_rfwd<T, N0, N1, 0><<<rplane_grid(npair), RP::TH, RP::smem, st>>>(r, ld, nband, band0, nullptr, RExx{}, AD, N2);
+    k_rzmul<T, N0, N1, N2><<<rz_grid(npair), RZ::TH, 0, st>>>(AD, reinterpret_cast<const T*>(c->teter_t.p), inv_nc);
+    k_rinv<T, N0, N1, false><<<rplane_grid(npair), RP::TH, RP::smem, st>>>(AD, out, ldo, nband, band0, accumulate, N2);
     PWB_CUDA(cudaGetLastError());
     return PW_OK;
   }
@@ -2207,9 +2033,6 @@ static int densgs_thunk(pw_ctx* c, const void* psi, int ld, int nband, int band0
                         double* rho, cudaStream_t st) {
   return Plan<T, N0, N1, N2>::density_gs_batch(c, (const T*)psi, ld, nband, band0, npair, w, rho, st);
 }
-template <typename T, int N0, int N1, int N2> static int vperm_thunk(pw_ctx* c, cudaStream_t st) {
-  return Plan<T, N0, N1, N2>::vperm_build(c, st);
-}
 template <typename T, int N0, int N1, int N2>
 static int buildqk_thunk(pw_ctx* c, const int* a, const double* b, const double* d, const long* e, const long* f,
                          const int* g, int n, const double* kv, void* out, cudaStream_t st) {
@@ -2229,7 +2052,6 @@ static int buildqk_thunk(pw_ctx* c, const int* a, const double* b, const double*
    {buildqk_thunk<double, a, b, c>, buildqk_thunk<float, a, b, c>},                                \
    {hpsikb_thunk<double, a, b, c>, hpsikb_thunk<float, a, b, c>},                                  \
    {hpsigs_thunk<double, a, b, c>, hpsigs_thunk<float, a, b, c>},                                  \
-   {densgs_thunk<double, a, b, c>, densgs_thunk<float, a, b, c>},                                  \
-   {vperm_thunk<double, a, b, c>, vperm_thunk<float, a, b, c>}}
+   {densgs_thunk<double, a, b, c>, densgs_thunk<float, a, b, c>}}
 
 }  // namespace pwb

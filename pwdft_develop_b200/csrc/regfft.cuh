@@ -1,0 +1,179 @@
+// Register-resident 1-D transforms for sm_100a.
+//
+// A transform of length N lives in the registers of P lanes, M = N / P
+// elements each: one lane up to 48 elements in FP32 (96 registers of data)
+// and 24 (or 30) in FP64, two lanes above.  Nothing goes through shared memory inside
+// a transform; the two-lane form exchanges M / 2 elements by shuffles for its
+// last (first) radix-2 stage.
+//
+//   fft_dit  in: v[m] = x[P m + p] (interleaved), out: v[j] = X[kout(p, j)]
+//   fft_dif  in: v[j] = X[kout(p, j)],            out: v[m] = x[P m + p]
+// Forward transforms take fft_dif and inverse ones fft_dit: on decaying spectra
+// that order rounds 2-8 % less at 60 and 72 than the other, and the two fit
+// together without a change of layout.
+//
+// Lanes of one transform are 16 apart (p = lane >> 4), so that each half-warp
+// walks 16 consecutive columns: full sectors in global memory and conflict-free
+// rows in shared memory.  All lanes of a warp must call a two-lane transform.
+#pragma once
+#include "fft.cuh"
+
+namespace pwb {
+
+template <typename T, int N> struct RegN {
+  static constexpr int P = N <= (sizeof(T) == 4 ? 48 : 24) || N == 30 ? 1 : 2;
+  static constexpr int M = N / P;
+  static constexpr int CW = 32 / P;    // transforms per warp
+  static constexpr bool OK = N % (2 * P) == 0 && M % 2 == 0 && M <= (sizeof(T) == 4 ? 48 : 36);
+  // register index j of lane p <-> frequency (kout) / sample P j + p (interleaved)
+  static __device__ __forceinline__ constexpr int kout(int p, int j) {
+    return P == 1 ? j : (j < M / 2 ? j : j + M / 2) + p * (M / 2);
+  }
+};
+
+__device__ __forceinline__ float2 shfl_x16(float2 v) {
+  return make_float2(__shfl_xor_sync(0xffffffffu, v.x, 16), __shfl_xor_sync(0xffffffffu, v.y, 16));
+}
+__device__ __forceinline__ double2 shfl_x16(double2 v) {
+  return make_double2(__shfl_xor_sync(0xffffffffu, v.x, 16), __shfl_xor_sync(0xffffffffu, v.y, 16));
+}
+template <typename V> __device__ __forceinline__ V csel(bool c, V a, V b) {
+  V r;
+  r.x = c ? a.x : b.x;
+  r.y = c ? a.y : b.y;
+  return r;
+}
+
+// A twiddle left on an input of the next butterfly: w v = kap u with
+// u = v + (tan or cot) i v, two FMAs instead of four products; the factor kap goes
+// into the butterfly's own FMAs.
+template <int R, int M_, int DIR, typename V> struct PendTw {
+  using T = typename RealOf<V>::t;
+  static constexpr int m = M_ % R;
+  static constexpr double c = TwR<R>::c[m], s = DIR * TwR<R>::s[m];
+  static constexpr bool big = (c < 0 ? -c : c) >= (s < 0 ? -s : s);
+  static constexpr double kap = big ? c : s;
+  static constexpr double t = big ? s / c : c / s;
+  static __device__ __forceinline__ V u(V v) {
+    if constexpr (big) {
+      if constexpr (t == 0) return v;
+      return mkc<V>(v.x - (T)t * v.y, v.y + (T)t * v.x);
+    } else {
+      if constexpr (t == 0) return mkc<V>(-v.y, v.x);
+      return mkc<V>((T)t * v.x - v.y, (T)t * v.y + v.x);
+    }
+  }
+};
+template <typename V> __device__ __forceinline__ V cfma(typename RealOf<V>::t k, V u, V a) {
+  return mkc<V>(a.x + k * u.x, a.y + k * u.y);
+}
+
+// In-place DFT of R elements in registers, natural order in and out, decimated
+// in time with the twiddles folded into the radix-4, -3 and -2 butterflies:
+// about 680 FP32 pipe operations at R = 48 against 800 of DFT<48>.
+template <int R, int DIR, typename V> struct RDFT {
+  using T = typename RealOf<V>::t;
+  static constexpr int B = R <= 5 ? R : (R % 4 == 0 ? 4 : (R % 3 == 0 ? 3 : (R % 2 == 0 ? 2 : 5)));
+  static constexpr int A = R / B;
+  static __device__ __forceinline__ void run(V* v) {
+    if constexpr (R <= 5) {
+      DFT<R, DIR, V>::run(v);
+    } else {
+      V t[R];
+      sfor<0, B>([&](auto bI) {
+        constexpr int b = decltype(bI)::value;
+        V a_[A];
+        sfor<0, A>([&](auto aI) { a_[decltype(aI)::value] = v[B * decltype(aI)::value + b]; });
+        RDFT<A, DIR, V>::run(a_);
+        sfor<0, A>([&](auto aI) { t[b * A + decltype(aI)::value] = a_[decltype(aI)::value]; });
+      });
+      sfor<0, A>([&](auto kI) {
+        constexpr int k = decltype(kI)::value;
+        if constexpr (B == 4) {
+          using P1 = PendTw<R, k, DIR, V>;
+          using P2 = PendTw<R, 2 * k, DIR, V>;
+          using P3 = PendTw<R, 3 * k, DIR, V>;
+          const V u1 = P1::u(t[A + k]), u2 = P2::u(t[2 * A + k]), u3 = P3::u(t[3 * A + k]);
+          const V a = cfma((T)P2::kap, u2, t[k]), b = cfma((T)-P2::kap, u2, t[k]);
+          constexpr double r = P3::kap / P1::kap;
+          const V s = cfma((T)r, u3, u1), d = cmuli<DIR>(cfma((T)-r, u3, u1));
+          v[k] = cfma((T)P1::kap, s, a);
+          v[k + 2 * A] = cfma((T)-P1::kap, s, a);
+          v[k + A] = cfma((T)P1::kap, d, b);
+          v[k + 3 * A] = cfma((T)-P1::kap, d, b);
+        } else if constexpr (B == 3) {
+          using P1 = PendTw<R, k, DIR, V>;
+          using P2 = PendTw<R, 2 * k, DIR, V>;
+          const V u1 = P1::u(t[A + k]), u2 = P2::u(t[2 * A + k]);
+          constexpr double r = P2::kap / P1::kap;
+          const V s = cfma((T)r, u2, u1), d = cmuli<DIR>(cfma((T)-r, u2, u1));
+          const V h = cfma((T)(-0.5 * P1::kap), s, t[k]);
+          constexpr double q = TwR<3>::s[1] * P1::kap;
+          v[k] = cfma((T)P1::kap, s, t[k]);
+          v[k + A] = cfma((T)q, d, h);
+          v[k + 2 * A] = cfma((T)-q, d, h);
+        } else if constexpr (B == 2) {
+          using P1 = PendTw<R, k, DIR, V>;
+          const V u1 = P1::u(t[A + k]);
+          v[k] = cfma((T)P1::kap, u1, t[k]);
+          v[k + A] = cfma((T)-P1::kap, u1, t[k]);
+        } else {
+          V c_[B];
+          sfor<0, B>([&](auto bI) {
+            constexpr int b = decltype(bI)::value;
+            c_[b] = twmul<R, b * k, DIR>(t[b * A + k]);
+          });
+          DFT<B, DIR, V>::run(c_);
+          sfor<0, B>([&](auto bI) { v[k + A * decltype(bI)::value] = c_[decltype(bI)::value]; });
+        }
+      });
+    }
+  }
+};
+
+// FUSE takes RDFT for the local part: 8 % faster where the FP32 / FP64 pipe binds
+// (the fine planes); the memory-bound passes gain nothing from it and keep DFT,
+// whose separately rounded twiddles are 10 % closer to the exact transform.
+template <typename T, int N, int DIR, bool FUSE = false> __device__ __forceinline__ void fft_dit(typename C2<T>::t* v, int p) {
+  using V = typename C2<T>::t;
+  using R = RegN<T, N>;
+  if constexpr (FUSE) RDFT<R::M, DIR, V>::run(v);
+  else DFT<R::M, DIR, V>::run(v);
+  if constexpr (R::P == 2) {
+    constexpr int H = R::M / 2;
+    const bool q = p != 0;
+    sfor<0, H>([&](auto jI) {
+      constexpr int j = decltype(jI)::value;
+      const V keep = csel(q, v[j + H], v[j]);
+      const V recv = shfl_x16(csel(q, v[j], v[j + H]));
+      const V e = csel(q, recv, keep);
+      V o = twmul<N, j, DIR>(csel(q, keep, recv));
+      o = csel(q, cmuli<DIR>(o), o);
+      v[j] = cadd(e, o);
+      v[j + H] = csub(e, o);
+    });
+  }
+}
+
+template <typename T, int N, int DIR, bool FUSE = false> __device__ __forceinline__ void fft_dif(typename C2<T>::t* v, int p) {
+  using V = typename C2<T>::t;
+  using R = RegN<T, N>;
+  if constexpr (R::P == 2) {
+    constexpr int H = R::M / 2;
+    const bool q = p != 0;
+    sfor<0, H>([&](auto jI) {
+      constexpr int j = decltype(jI)::value;
+      const V a = cadd(v[j], v[j + H]);
+      V b = twmul<N, j, DIR>(csub(v[j], v[j + H]));
+      b = csel(q, cmuli<DIR>(b), b);
+      const V recv = shfl_x16(csel(q, a, b));
+      const V keep = csel(q, b, a);
+      v[j] = csel(q, recv, keep);
+      v[j + H] = csel(q, keep, recv);
+    });
+  }
+  if constexpr (FUSE) RDFT<R::M, DIR, V>::run(v);
+  else DFT<R::M, DIR, V>::run(v);
+}
+
+}  // namespace pwb
