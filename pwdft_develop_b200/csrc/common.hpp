@@ -214,6 +214,8 @@ struct pw_ctx {
   std::vector<cudaEvent_t> ev_pool;
   // scratch for the band-pair pipeline
   int pair_cap = 0;
+  bool batch_set = false;          // pw_set_band_batch was called: the batch stays as set
+  bool captured = false;           // a stream capture has recorded this context's scratch
   pwb::DevBuf s_ad, s_k, s_bc, s_wp, s_w;
   pwb::DevBuf s_host_in, s_host_out;   // device staging for the host-pointer entry points
   pwb::DevBuf gs_full_idx, gs_exx_tw;   // G-space exchange: full-grid index of G_s and -G_s, N-point twiddles

@@ -204,6 +204,37 @@ int ensure_scratch(pw_ctx* c, int npair) {
   return PW_OK;
 }
 
+// The band batch follows the calls: one launch per pass over all `npair` fields
+// where the batch fields fit in 1 GiB (Si64, 80 pairs: the five passes take
+// 400 us in one batch and 436 us in batches of 32, and the projector matrix
+// is read once, not three times).  It stays as it is once the caller has set it
+// and once a capture has recorded the buffers.  The passes then split the
+// bands evenly.
+int batch_pairs(pw_ctx* c, int npair, cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+    cudaGetLastError();
+    cs = cudaStreamCaptureStatusActive;
+  }
+  if (cs != cudaStreamCaptureStatusNone) c->captured = true;
+  if (npair > c->pair_cap && !c->batch_set && !c->captured) {
+    const size_t per = (2 * (size_t)c->ntot + (size_t)c->nf[2] * (c->n[1] + 1) * (c->n[0] + 1)) * 2 * c->esz;
+    const int want = (int)std::min<size_t>(npair, ((size_t)1 << 30) / per), old = c->pair_cap;
+    if (want > old) {
+      // other streams may still run passes on the present buffers; cudaFree waits for them
+      c->pair_cap = 0;
+      if (ensure_scratch(c, want)) {
+        cudaGetLastError();
+        c->pair_cap = 0;
+        if (ensure_scratch(c, old)) return 0;
+        c->batch_set = true;     // no room: keep the old batch
+      }
+    }
+  }
+  const int nb = (npair + c->pair_cap - 1) / std::max(1, c->pair_cap);
+  return c->pair_cap < 1 ? 0 : (npair + nb - 1) / std::max(1, nb);
+}
+
 }  // namespace pwb
 
 using namespace pwb;
@@ -366,6 +397,7 @@ int pw_set_band_batch(pw_ctx* ctx, int nband_batch) {
   PWB_CHECK(ctx && nband_batch > 0, PW_EINVAL, "bad band batch");
   PWB_CUDA(cudaSetDevice(ctx->device));
   ctx->pair_cap = 0;
+  ctx->batch_set = true;
   return ensure_scratch(ctx, (nband_batch + 1) / 2);
 }
 
@@ -563,7 +595,9 @@ int pw_hpsi(pw_ctx* ctx, const void* psi, int ld, void* hpsi, int ldh, int nband
     int rc = prepare_wfn_filter(ctx);
     if (rc) return rc;
   }
-  const int cap = ctx->pair_cap;
+  if (nband == 0) return PW_OK;
+  const int cap = batch_pairs(ctx, (nband + 1) / 2, st);
+  if (cap < 1) return PW_ENOMEM;
   for (int b0 = 0; b0 < nband; b0 += 2 * cap) {
     const int npair = std::min(cap, (nband - b0 + 1) / 2);
     int rc = run_hpsi(ctx, psi, ld, hpsi, ldh, nband, b0, npair, accumulate, st);
@@ -643,7 +677,9 @@ int pw_teter_precond(pw_ctx* ctx, const void* r, int ld, void* w, int ldw, int n
   PWB_CHECK(nband >= 0 && ld >= ctx->ntot && ldw >= ctx->ntot, PW_EINVAL, "Domain size does not match.");
   PWB_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t st = (cudaStream_t)stream;
-  const int cap = ctx->pair_cap;
+  if (nband == 0) return PW_OK;
+  const int cap = batch_pairs(ctx, (nband + 1) / 2, st);
+  if (cap < 1) return PW_ENOMEM;
   for (int b0 = 0; b0 < nband; b0 += 2 * cap) {
     const int npair = std::min(cap, (nband - b0 + 1) / 2);
     int rc = run_teter(ctx, r, ld, w, ldw, nband, b0, npair, accumulate, st);
