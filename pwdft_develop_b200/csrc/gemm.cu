@@ -96,10 +96,10 @@ __global__ void k_wait_probe(unsigned long long limit_ns) {
   atomicCAS(&g_gemm_error, 0, 7);
 }
 
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y) {
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y)
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(smem_u32(dst)), "l"(map), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
 
@@ -154,6 +154,8 @@ struct GemmArgs {
   int accumulate;        // epi 1 / 2: C += tile
   int sym;               // symmetric product (A = B): only tiles not strictly below the diagonal
   int ntiles;            // sym: number of those tiles
+  int nbatch;            // products of this shape
+  long bs_c;             // epi 1 / 2: elements of C from one product to the next
 };
 
 // tiles of column block nt that are not strictly below the diagonal of a
@@ -187,7 +189,8 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CU
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tilesM = (g.M + GM - 1) / GM, tilesN = (g.N + BN - 1) / BN;
-  const int total = (g.sym ? g.ntiles : tilesM * tilesN) * g.nsplit;
+  const int per = (g.sym ? g.ntiles : tilesM * tilesN) * g.nsplit;   // tiles of one product
+  const int total = per * g.nbatch;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < SM::NSTAGE; ++s) {
@@ -212,8 +215,13 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CU
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = *tmem_slot;
 
-  auto coords = [&](int t, int& m0, int& n0, int& split, int& kbeg, int& nkb) {
+  auto coords = [&](int t, int& m0, int& n0, int& split, int& kbeg, int& nkb, int& bt) {
     int mt, ntl;
+    bt = 0;
+    if (g.nbatch > 1) {
+      bt = t / per;
+      t -= bt * per;
+    }
     if (g.sym) {
       // the upper tiles, column block by column block
       int idx = t % g.ntiles;
@@ -242,8 +250,8 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CU
       long it = 0;
       bool stop = false;
       for (int t = blockIdx.x; t < total && !stop; t += gridDim.x) {
-        int m0, n0, split, kbeg, nkb;
-        coords(t, m0, n0, split, kbeg, nkb);
+        int m0, n0, split, kbeg, nkb, bt;
+        coords(t, m0, n0, split, kbeg, nkb, bt);
         for (int kb = 0; kb < nkb; ++kb) {
           const int s = (int)(it % SM::NSTAGE);
           if (it >= SM::NSTAGE && !mbar_wait(&empty[s], (uint32_t)(((it / SM::NSTAGE) - 1) & 1), 1)) {
@@ -255,10 +263,10 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CU
           unsigned char* st = base + s * SM::STAGE;
           mbar_expect_tx(&full[s], SM::STAGE);
           const int kx = kbeg + kb * GK;
-          tma_load_2d(st, &tmA_hi, &full[s], kx, m0);
-          tma_load_2d(st + SM::A_BYTES, &tmA_lo, &full[s], kx, m0);
-          tma_load_2d(st + 2 * SM::A_BYTES, &tmB_hi, &full[s], kx, n0);
-          tma_load_2d(st + 2 * SM::A_BYTES + SM::B_BYTES, &tmB_lo, &full[s], kx, n0);
+          tma_load_3d(st, &tmA_hi, &full[s], kx, m0, bt);
+          tma_load_3d(st + SM::A_BYTES, &tmA_lo, &full[s], kx, m0, bt);
+          tma_load_3d(st + 2 * SM::A_BYTES, &tmB_hi, &full[s], kx, n0, bt);
+          tma_load_3d(st + 2 * SM::A_BYTES + SM::B_BYTES, &tmB_lo, &full[s], kx, n0, bt);
           ++it;
         }
       }
@@ -273,8 +281,8 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CU
       int lt = 0;
       bool ok = true, any = false;
       for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++lt) {
-        int m0, n0, split, kbeg, nkb;
-        coords(t, m0, n0, split, kbeg, nkb);
+        int m0, n0, split, kbeg, nkb, bt;
+        coords(t, m0, n0, split, kbeg, nkb, bt);
         const int buf = lt & 1;
         if (lt >= 2 && !mbar_wait(&tempty[buf], (uint32_t)(((lt >> 1) - 1) & 1), 5)) { ok = false; break; }
         asm volatile("tcgen05.fence::after_thread_sync;");
@@ -314,8 +322,8 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CU
     const int q = warp & 3;
     int lt = 0;
     for (int t = blockIdx.x; t < total; t += gridDim.x, ++lt) {
-      int m0, n0, split, kbeg, nkb;
-      coords(t, m0, n0, split, kbeg, nkb);
+      int m0, n0, split, kbeg, nkb, bt;
+      coords(t, m0, n0, split, kbeg, nkb, bt);
       const int buf = lt & 1;
       int ok = 1;
       if (lane == 0) ok = mbar_wait(&tfull[buf], (uint32_t)((lt >> 1) & 1), 4) ? 1 : 0;
@@ -330,13 +338,13 @@ k_gemm_tn(const __grid_constant__ CUtensorMap tmA_hi, const __grid_constant__ CU
         float* dst;
         long cs;                            // column stride of the destination
         if (g.epi == 0) {
-          dst = g.ws + ((long)split * g.N + n0 + c0) * g.M + row;
+          dst = g.ws + (((long)bt * g.nsplit + split) * g.N + n0 + c0) * g.M + row;
           cs = g.M;
         } else if (g.epi == 2) {
-          dst = g.C + (long)(n0 + c0) * g.ldc + row;
+          dst = g.C + bt * g.bs_c + (long)(n0 + c0) * g.ldc + row;
           cs = g.ldc;
         } else {
-          dst = g.C + (long)row * g.ldc + n0 + c0;
+          dst = g.C + bt * g.bs_c + (long)row * g.ldc + n0 + c0;
           cs = 1;
         }
         float cv[32];
@@ -442,7 +450,8 @@ __global__ void k_split_bf16_t(const float* __restrict__ x, long ld_in, int ncol
 // scale, written as double or float, directly or transposed.
 __global__ void k_splitk_reduce(const float* __restrict__ ws, int nsplit, int M, int N, const float* __restrict__ rs,
                                 const float* __restrict__ cs, int transpose, int out_f64, void* out, long ldo,
-                                __nv_bfloat16* bhi, __nv_bfloat16* blo, long ldb, int sym_bn) {
+                                __nv_bfloat16* bhi, __nv_bfloat16* blo, long ldb, int sym_bn, long bs_bf) {
+  ws += (long)blockIdx.y * nsplit * M * N;   // one product of a batch
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= (long)M * N) return;
   const int n = (int)(i / M), m = (int)(i - (long)n * M);
@@ -469,7 +478,7 @@ __global__ void k_splitk_reduce(const float* __restrict__ ws, int nsplit, int M,
     else reinterpret_cast<float*>(out)[o] = (float)s;
   }
   if (bhi) {
-    const long ob = transpose ? (long)n * ldb + m : (long)m * ldb + n;
+    const long ob = blockIdx.y * bs_bf + (transpose ? (long)n * ldb + m : (long)m * ldb + n);
     const float v = (float)s;
     const __nv_bfloat16 h = __float2bfloat16_rn(v);
     bhi[ob] = h;
@@ -492,16 +501,18 @@ static PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
   return fn;
 }
 
-// 2-D bf16 tensor map over rows x K (K contiguous, row stride ld elements), box GK x box_rows
-static int make_tmap(CUtensorMap* m, const void* ptr, long rows, long K, long ld, int box_rows) {
+// bf16 tensor map over batch x rows x K (K contiguous, row stride ld, batch stride bs elements), box GK x box_rows
+static int make_tmap(CUtensorMap* m, const void* ptr, long rows, long K, long ld, int box_rows, int nbatch, long bs) {
   auto enc = get_encode();
   PWB_CHECK(enc, PW_ECUDA, "cuTensorMapEncodeTiled unavailable");
-  PWB_CHECK(((uintptr_t)ptr & 15) == 0 && (ld * 2) % 16 == 0, PW_EINVAL, "TMA operand not 16-byte aligned");
-  cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)(ld * 2)};
-  cuuint32_t box[2] = {(cuuint32_t)GK, (cuuint32_t)box_rows};
-  cuuint32_t es[2] = {1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es,
+  if (nbatch == 1) bs = rows * ld;
+  PWB_CHECK(((uintptr_t)ptr & 15) == 0 && (ld * 2) % 16 == 0 && (bs * 2) % 16 == 0, PW_EINVAL,
+            "TMA operand not 16-byte aligned");
+  cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)nbatch};
+  cuuint64_t strides[2] = {(cuuint64_t)(ld * 2), (cuuint64_t)(bs * 2)};
+  cuuint32_t box[3] = {(cuuint32_t)GK, (cuuint32_t)box_rows, 1};
+  cuuint32_t es[3] = {1, 1, 1};
+  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, es,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   PWB_CHECK(r == CUDA_SUCCESS, PW_ECUDA, "cuTensorMapEncodeTiled failed");
@@ -528,8 +539,10 @@ template <int BN> static int launch_bn(const SplitOperand& A, const SplitOperand
   }
   CUtensorMap ah, al, bh, bl;
   int rc;
-  if ((rc = make_tmap(&ah, A.hi, A.rows, g.K, A.ld, GM)) || (rc = make_tmap(&al, A.lo, A.rows, g.K, A.ld, GM)) ||
-      (rc = make_tmap(&bh, B.hi, B.rows, g.K, B.ld, BN)) || (rc = make_tmap(&bl, B.lo, B.rows, g.K, B.ld, BN)))
+  if ((rc = make_tmap(&ah, A.hi, A.rows, g.K, A.ld, GM, g.nbatch, A.bs)) ||
+      (rc = make_tmap(&al, A.lo, A.rows, g.K, A.ld, GM, g.nbatch, A.bs)) ||
+      (rc = make_tmap(&bh, B.hi, B.rows, g.K, B.ld, BN, g.nbatch, B.bs)) ||
+      (rc = make_tmap(&bl, B.lo, B.rows, g.K, B.ld, BN, g.nbatch, B.bs)))
     return rc;
   GemmArgs ga = g;
   ga.nsplit = nsplit;
@@ -538,7 +551,7 @@ template <int BN> static int launch_bn(const SplitOperand& A, const SplitOperand
     ga.ntiles = 0;
     for (int nt = 0; nt < tilesN; ++nt) ga.ntiles += sym_tiles_in_col(nt, BN, tilesM);
   }
-  const long total = (long)(ga.sym ? ga.ntiles : tilesM * tilesN) * nsplit;
+  const long total = (long)(ga.sym ? ga.ntiles : tilesM * tilesN) * nsplit * ga.nbatch;
   const int grid = (int)std::min<long>(total, num_sms());
   k_gemm_tn<BN><<<grid, GEMM_THREADS, SM::BYTES, st>>>(ah, al, bh, bl, ga);
   PWB_CUDA(cudaGetLastError());
@@ -614,7 +627,7 @@ int split_bf16_t(const float* x, long ld_in, int ncol, int nrow, void* hi, void*
 }
 
 int gemm_tn_reduce(const SplitOperand& A, const SplitOperand& B, int K, int nterms, DevBuf& ws,
-                   const ReduceOut& out, cudaStream_t st, int bn, int sym) {
+                   const ReduceOut& out, cudaStream_t st, int bn, int sym, int nbatch) {
   const int M = A.rows, N = B.rows;
   if (M == 0 || N == 0) return PW_OK;
   const int BN = bn > 0 ? bn : pick_bn(N);
@@ -624,6 +637,7 @@ int gemm_tn_reduce(const SplitOperand& A, const SplitOperand& B, int K, int nter
     tiles = 0;
     for (int nt = 0; nt < (N + BN - 1) / BN; ++nt) tiles += sym_tiles_in_col(nt, BN, (M + GM - 1) / GM);
   }
+  tiles *= nbatch;
   // enough CTAs to fill the GPU twice over, each with >= 4 K-blocks
   int nsplit = std::max(1, (2 * num_sms() + tiles - 1) / tiles);
   const int maxsplit = std::max(1, (K + 4 * GK - 1) / (4 * GK));
@@ -636,29 +650,30 @@ int gemm_tn_reduce(const SplitOperand& A, const SplitOperand& B, int K, int nter
   nsplit = std::max(nsplit, (K + KCHUNK_MAX - 1) / KCHUNK_MAX);
   int kchunk = ((K + nsplit - 1) / nsplit + GK - 1) / GK * GK;
   nsplit = (K + kchunk - 1) / kchunk;
-  int rc = ws.alloc((size_t)nsplit * M * N * sizeof(float));
+  int rc = ws.alloc((size_t)nbatch * nsplit * M * N * sizeof(float));
   if (rc) return rc;
   GemmArgs g{};
   g.M = M; g.N = N; g.K = K; g.kchunk = kchunk; g.nterms = nterms; g.epi = 0;
   g.ws = reinterpret_cast<float*>(ws.p);
   g.sym = sym;
+  g.nbatch = nbatch;
   if ((rc = launch(A, B, g, BN, nsplit, st))) return rc;
   const long tot = (long)M * N;
-  k_splitk_reduce<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(
+  k_splitk_reduce<<<dim3((unsigned)((tot + 255) / 256), nbatch), 256, 0, st>>>(
       g.ws, nsplit, M, N, out.row_scale, out.col_scale, out.transpose, out.f64, out.out, out.ldo,
-      (__nv_bfloat16*)out.bf_hi, (__nv_bfloat16*)out.bf_lo, out.ldb, sym ? BN : 0);
+      (__nv_bfloat16*)out.bf_hi, (__nv_bfloat16*)out.bf_lo, out.ldb, sym ? BN : 0, out.bs_bf);
   PWB_CUDA(cudaGetLastError());
   return PW_OK;
 }
 
 int gemm_tn_store(const SplitOperand& A, const SplitOperand& B, int K, int nterms, float* C, long ldc, int accumulate,
-                  cudaStream_t st, int transposed, int bn) {
+                  cudaStream_t st, int transposed, int bn, int nbatch, long bs_c) {
   const int M = A.rows, N = B.rows;
   if (M == 0 || N == 0) return PW_OK;
   const int BN = bn > 0 ? bn : (N >= 256 ? 256 : pick_bn(N));
   GemmArgs g{};
   g.M = M; g.N = N; g.K = K; g.kchunk = ((K + GK - 1) / GK) * GK; g.nterms = nterms; g.epi = transposed ? 2 : 1;
-  g.C = C; g.ldc = ldc; g.accumulate = accumulate;
+  g.C = C; g.ldc = ldc; g.accumulate = accumulate; g.nbatch = nbatch; g.bs_c = bs_c;
   return launch(A, B, g, BN, 1, st);
 }
 

@@ -210,8 +210,9 @@ int pw_hpsi_kbatch(pw_ctx* ctx, const void* psi, int ld, void* hpsi, int ldh, in
   cudaStream_t st = (cudaStream_t)stream;
   const int nf = ctx->nkb * nband;
   if (nf == 0) return PW_OK;
-  const int cap = batch_pairs(ctx, nf, st);
+  int cap = batch_pairs(ctx, nf, st);
   if (cap < 1) return PW_ENOMEM;
+  if (cap > nband) cap -= cap % nband;   // whole k-points per batch
   for (int f0 = 0; f0 < nf; f0 += cap) {
     const int n = std::min(cap, nf - f0);
     int rc = run_hpsi_kbatch(ctx, psi, ld, hpsi, ldh, f0, n, accumulate, st, nband, ctx->ekin_kb.p,

@@ -1721,6 +1721,13 @@ struct Plan {
     // V_nl psi = Q diag(d) Q^H psi with the complex coarse projector matrix Q of
     // each k-point, one GEMM pair per k segment of the batch
     const size_t kq_per = kq_bf_bytes(c);
+    if constexpr (std::is_same<T, float>::value) {
+      // whole k-points of one batch together
+      const void* q0 = qk_all && c->qkb_bf.p ? (const char*)c->qkb_bf.p + (size_t)(band0 / fpk) * kq_per : nullptr;
+      if (q0 && band0 % fpk == 0 && nb % fpk == 0)
+        return nl_k_tc(c, q0, reinterpret_cast<const float*>(psi + (long)band0 * ld), ld,
+                       reinterpret_cast<float*>(out + (long)band0 * ldo), ldo, fpk, nb / fpk, st);
+    }
     for (int f = band0; f < band0 + nb;) {
       const int kk = f / fpk;
       const int f1 = (int)std::min<long>(band0 + nb, (long)(kk + 1) * fpk);
@@ -1737,7 +1744,9 @@ struct Plan {
   // interleaved (re, im) view.  [Re W; Im W] = d o (A1 psi) (K = 2 ntot, split-K
   // reduced, written as the bf16 operand of the next product), then
   // psi_out += A2 [Re W; Im W] (K = 2 nproj) on the grid-major rows.
-  static int nl_k_tc(pw_ctx* c, const void* qbf, const float* x, int ld, float* y, int ldo, int nb, cudaStream_t st) {
+  // nk k-points (their operands kq_bf_bytes apart) of nb bands each in one launch per step.
+  static int nl_k_tc(pw_ctx* c, const void* qbf, const float* x, int ld, float* y, int ldo, int nb, int nk,
+                     cudaStream_t st) {
     const int np = c->nproj, np2 = c->nkp2;
     const long nt = c->ntot, nt2 = 2 * nt;
     const char* a1h = (const char*)qbf;
@@ -1745,27 +1754,31 @@ struct Plan {
     const char* a2h = a1l + (size_t)2 * np * nt2 * 2;
     const char* a2l = a2h + (size_t)nt2 * np2 * 2;
     int rc;
-    if ((rc = c->s_psi_bf.alloc((size_t)2 * nb * nt2 * 2))) return rc;
-    if ((rc = c->s_w_bf.alloc((size_t)2 * nb * np2 * 2))) return rc;
+    const size_t nf = (size_t)nk * nb;
+    const long kstep = (long)(kq_bf_bytes(c) / 2);
+    if ((rc = c->s_psi_bf.alloc(2 * nf * nt2 * 2))) return rc;
+    if ((rc = c->s_w_bf.alloc(2 * nf * np2 * 2))) return rc;
     char* pb = (char*)c->s_psi_bf.p;
     char* wb = (char*)c->s_w_bf.p;
-    PWB_CUDA(cudaMemsetAsync(wb, 0, (size_t)2 * nb * np2 * 2, st));
     { Launch L_(c, st, KK_MISC);
-    if ((rc = split_bf16(x, 2L * ld, (int)nt2, nb, pb, pb + (size_t)nb * nt2 * 2, nt2, 1.0f, st))) return rc; }
-    SplitOperand A{a1h, a1l, 2 * np, nt2};
-    SplitOperand B{pb, pb + (size_t)nb * nt2 * 2, nb, nt2};
+    if ((rc = split_bf16(x, 2L * ld, (int)nt2, (int)nf, pb, pb + nf * nt2 * 2, nt2, 1.0f, st))) return rc; }
+    SplitOperand A{a1h, a1l, 2 * np, nt2, kstep};
+    SplitOperand B{pb, pb + nf * nt2 * 2, nb, nt2, (long)nb * nt2};
     ReduceOut ro;
     ro.transpose = 1;
     ro.row_scale = reinterpret_cast<const float*>(c->qdk2.p);
     ro.bf_hi = wb;
-    ro.bf_lo = wb + (size_t)nb * np2 * 2;
+    ro.bf_lo = wb + nf * np2 * 2;
     ro.ldb = np2;
+    ro.bs_bf = (long)nb * np2;
     { Launch L_(c, st, KK_GRAM);
-    if ((rc = gemm_tn_reduce(A, B, (int)nt2, c->gemm_terms, c->s_ws, ro, st, c->gemm_bn))) return rc; }
-    SplitOperand W{wb, wb + (size_t)nb * np2 * 2, nb, np2};
-    SplitOperand QT{a2h, a2l, (int)nt2, np2};
+    if ((rc = gemm_tn_reduce(A, B, (int)nt2, c->gemm_terms, c->s_ws, ro, st, c->gemm_bn, 0, nk))) return rc; }
+    // the bf16 rows end at 2 np of np2: the tensor maps stop there, the pad is never read
+    SplitOperand W{wb, wb + nf * np2 * 2, nb, np2, (long)nb * np2};
+    SplitOperand QT{a2h, a2l, (int)nt2, np2, kstep};
     { Launch L_(c, st, KK_GRAM);
-    if ((rc = gemm_tn_store(QT, W, 2 * np, c->gemm_terms, y, 2L * ldo, 1, st, 1, c->gemm_bn_store))) return rc; }
+    if ((rc = gemm_tn_store(QT, W, 2 * np, c->gemm_terms, y, 2L * ldo, 1, st, 1, c->gemm_bn_store, nk,
+                            2L * ldo * nb))) return rc; }
     return PW_OK;
   }
 
@@ -1774,7 +1787,7 @@ struct Plan {
     int rc;
     if constexpr (std::is_same<T, float>::value) {
       if (!qbf) { set_error("k-point projector bf16 copies missing"); return PW_ENOTREADY; }
-      return nl_k_tc(c, qbf, reinterpret_cast<const float*>(x), ld, reinterpret_cast<float*>(y), ldo, nb, st);
+      return nl_k_tc(c, qbf, reinterpret_cast<const float*>(x), ld, reinterpret_cast<float*>(y), ldo, nb, 1, st);
     } else {
     cublasHandle_t h = (cublasHandle_t)c->blas;
     if (cublasSetStream(h, st) != CUBLAS_STATUS_SUCCESS) { set_error("cublasSetStream failed"); return PW_ECUDA; }

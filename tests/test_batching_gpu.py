@@ -1,0 +1,83 @@
+"""Batch rules: the band batch that follows the call (growth, even split, frozen
+by a capture or by the caller) and the k-point projector products batched over
+whole k-points.  The same kernels run on every batch shape, so results agree to
+the bit where only the batch changes; FP32 k-points against one k at a time
+differ by the split-K partition of the projector sums (1e-5, the FP32 bar)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+A = 10.26
+
+
+def _ctx(prec, n=(16, 16, 16), **kw):
+    from oracle import pw
+    from pwdft_develop_b200 import Context
+    L, z, pos = pw.make_crystal("Si", (1, 1, 1), A, 0.02, 77)
+    c = Context(L, n, tuple(2 * x for x in n), precision=prec)
+    c.set_atoms([z] * len(pos), pos)
+    rng = np.random.default_rng(3)
+    c.set_vtot(rng.uniform(-1, 0.5, c.ntotFine))
+    return c
+
+
+def _rand(c, nb, seed=5):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn((nb, c.ntot), generator=g, device="cuda", dtype=torch.float64).to(c.torch_dtype)
+
+
+@pytest.mark.parametrize("nb", [1, 64, 65, 150, 307])
+def test_batch_follows_the_call(nb):
+    import torch
+    c, d = _ctx("f64"), _ctx("f64")
+    d.set_band_batch(14)
+    x = _rand(c, nb)
+    ref = torch.cat([c.teter(x[i:i + 2]) for i in range(0, nb, 2)])
+    assert torch.equal(c.teter(x), ref)
+    assert torch.equal(d.teter(x), ref)
+    # the FP64 projector products are a library's: equal to rounding only
+    a, b = c.hpsi(x), d.hpsi(x)
+    assert (a - b).abs().max() <= 1e-13 * a.abs().max()
+
+
+def test_a_captured_call_outlives_larger_ones():
+    import torch
+    c = _ctx("f32")
+    x = _rand(c, 7)
+    out = torch.empty_like(x)
+    g = c.capture_hpsi(x, out)
+    g.replay()
+    torch.cuda.synchronize()
+    ref = out.clone()
+    big = _rand(c, 200, seed=9)
+    y = c.hpsi(big)
+    assert torch.isfinite(y).all()
+    out.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("batch", [None, 2, 10, 22, 30])
+def test_kpoint_batches(prec, batch):
+    """nk = 5 of nb = 7: all together, whole k-points per batch (22, 30 fields)
+    and k-points cut by the batch (1, 5 fields)."""
+    import torch
+    c = _ctx(prec)
+    if batch:
+        c.set_band_batch(2 * batch)
+    rng = np.random.default_rng(1)
+    ks = rng.uniform(-0.3, 0.3, (5, 3))
+    c.set_kpoints(ks)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    ct = torch.complex128 if prec == "f64" else torch.complex64
+    x = torch.randn((5, 7, c.ntot, 2), generator=g, device="cuda", dtype=torch.float64)
+    x = torch.view_as_complex(x).to(ct)
+    got = c.hpsi_kbatch(x)
+    for i, k in enumerate(ks):
+        c.set_kpoint(k)
+        ref = c.hpsi_k(x[i].contiguous())
+        err = (got[i] - ref).abs().max() / ref.abs().max()
+        assert err <= (1e-5 if prec == "f32" else 1e-13), (i, float(err))
