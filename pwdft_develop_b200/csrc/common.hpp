@@ -46,10 +46,12 @@ struct PerDeviceOnce {
   void mark() { bits.fetch_or(1ull << dev(), std::memory_order_release); }
 };
 
-// Device buffer owned by a context.
+// Device buffer owned by a context.  With `keep` set, a block outgrown by a
+// later call goes there instead of being freed (a captured graph still reads it).
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  std::vector<void*>* keep = nullptr;
   int alloc(size_t nbytes);
   void release();
   ~DevBuf() { release(); }
@@ -216,6 +218,14 @@ struct pw_ctx {
   int pair_cap = 0;
   bool batch_set = false;          // pw_set_band_batch was called: the batch stays as set
   bool captured = false;           // a stream capture has recorded this context's scratch
+  std::vector<void*> retired;      // outgrown blocks that a captured graph may still use; freed with the context
+  void mark_captured() {
+    if (captured) return;
+    captured = true;
+    for (pwb::DevBuf* b : {&s_ad, &s_k, &s_bc, &s_wp, &s_w, &s_wq, &s_psi_bf, &s_w_bf, &s_ws, &s_gx_bf, &s_gy_bf, &s_rot,
+                           &s_rot_x, &s_exx, &gsx_psir, &gsx_phir, &gsx_acc, &gsx_fields})
+      b->keep = &retired;
+  }
   pwb::DevBuf s_ad, s_k, s_bc, s_wp, s_w;
   pwb::DevBuf s_host_in, s_host_out;   // device staging for the host-pointer entry points
   pwb::DevBuf gs_full_idx, gs_exx_tw;   // G-space exchange: full-grid index of G_s and -G_s, N-point twiddles

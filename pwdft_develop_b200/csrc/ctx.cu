@@ -19,6 +19,11 @@ void set_error(const std::string& msg) { g_err = msg; }
 
 int DevBuf::alloc(size_t nbytes) {
   if (nbytes <= bytes && p) return PW_OK;
+  if (p && keep) {
+    keep->push_back(p);
+    p = nullptr;
+    bytes = 0;
+  }
   release();
   if (nbytes == 0) return PW_OK;
   cudaError_t e = cudaMalloc(&p, nbytes);
@@ -216,7 +221,7 @@ int batch_pairs(pw_ctx* c, int npair, cudaStream_t st) {
     cudaGetLastError();
     cs = cudaStreamCaptureStatusActive;
   }
-  if (cs != cudaStreamCaptureStatusNone) c->captured = true;
+  if (cs != cudaStreamCaptureStatusNone) c->mark_captured();
   if (npair > c->pair_cap && !c->batch_set && !c->captured) {
     const size_t per = (2 * (size_t)c->ntot + (size_t)c->nf[2] * (c->n[1] + 1) * (c->n[0] + 1)) * 2 * c->esz;
     const int want = (int)std::min<size_t>(npair, ((size_t)1 << 30) / per), old = c->pair_cap;
@@ -325,6 +330,7 @@ int pw_ctx_destroy(pw_ctx* ctx) {
   if (ctx->nl_join) cudaEventDestroy(ctx->nl_join);
   if (ctx->scf_cache_free) ctx->scf_cache_free(ctx->scf_cache);
   if (ctx->twin) pw_ctx_destroy(ctx->twin);
+  for (void* p : ctx->retired) cudaFree(p);
   delete ctx;
   return PW_OK;
 }

@@ -1420,8 +1420,11 @@ struct Plan {
     const int ntx = (N0 + TX - 1) / TX;
     // dense projector mode: Q D Q^T psi depends on psi only, so its GEMMs run
     // on a second stream while the FFT chain runs (their first output goes to
-    // the rows of out, which k_cxy_inv then accumulates into after the join);
-    // with pw_profile on they run after it, so each kernel is timed alone
+    // the rows of out, which the last coarse pass then accumulates into after
+    // the join), for all bands of the call at once: Q is read once per call, not
+    // once per batch (Si216, 480 bands: Q is 1.6 GB).  The split bands take at
+    // most 1 GiB at a time.  With pw_profile on the products run batch by batch
+    // after the chain, so each kernel is timed alone
     const int nbnl = std::min(2 * npair, nband - band0);
     const bool dense_nl = c->nl_mode == PW_NL_DENSE && c->have_nl && c->nproj > 0 && nbnl > 0;
     cudaStream_t sn = nullptr;
@@ -1430,14 +1433,18 @@ struct Plan {
       if (!c->nl_fork) PWB_CUDA(cudaEventCreateWithFlags(&c->nl_fork, cudaEventDisableTiming));
       if (!c->nl_join) PWB_CUDA(cudaEventCreateWithFlags(&c->nl_join, cudaEventDisableTiming));
       sn = c->nl_st;
-      PWB_CUDA(cudaEventRecord(c->nl_fork, st));
-      PWB_CUDA(cudaStreamWaitEvent(sn, c->nl_fork, 0));
-      if ((rc = dense_apply(c, nl_set(c, filt), psi + (long)band0 * ld, ld, out + (long)band0 * ldo, ldo, nbnl, sn,
-                            accumulate))) {
-        cudaStreamWaitEvent(st, c->nl_fork, 0);
-        return rc;
+      if (band0 == 0) {
+        PWB_CUDA(cudaEventRecord(c->nl_fork, st));
+        PWB_CUDA(cudaStreamWaitEvent(sn, c->nl_fork, 0));
+        const int group = (int)std::max<long>(1, (1L << 30) / (4 * (long)c->ntot));
+        for (int g0 = 0; g0 < nband; g0 += group)
+          if ((rc = dense_apply(c, nl_set(c, filt), psi + (long)g0 * ld, ld, out + (long)g0 * ldo, ldo,
+                                std::min(group, nband - g0), sn, accumulate))) {
+            cudaStreamWaitEvent(st, c->nl_fork, 0);
+            return rc;
+          }
+        PWB_CUDA(cudaEventRecord(c->nl_join, sn));
       }
-      PWB_CUDA(cudaEventRecord(c->nl_join, sn));
     }
     if (reg(c) && c->nl_mode == PW_NL_DENSE) {
       reg_up<0>(c, psi, ld, nband, band0, npair, reinterpret_cast<const T*>(c->ekin_t.p), 0, 1 << 30, 0, st);
