@@ -132,6 +132,12 @@ template <typename X> static int upload(DevBuf& b, const std::vector<X>& h) {
   return PW_OK;
 }
 
+// one of the four interleaved columns (VAL, DX, DY, DZ) of n projector points
+__global__ void k_pick_column(const double* __restrict__ val4, long n, int col, double* __restrict__ out) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    out[i] = val4[4 * i + col];
+}
+
 static int local_part(pw_ctx* ctx, const double* rho, double* F_dev) {
   const long nf = ctx->ntotf;
   const int natom = (int)ctx->atom_z.size();
@@ -192,29 +198,44 @@ static int nl_contract(pw_ctx* ctx, const double* psi, int ld, int nb, const std
   for (int a = 0; a < natom; ++a) aoff[a + 1] += aoff[a];
   std::vector<double> gl(np);
   for (int l = 0; l < np; ++l) gl[l] = ctx->h_pgamma[l] * ctx->vol / (double)nt;
-  std::vector<double> dcol[3];
+  // the analytic columns go to the device interleaved, as pw_set_atoms holds
+  // them, and are picked apart there (a host loop over the 14 M values of Si64
+  // took 100 of 133 ms)
+  DevBuf d_val4;
+  const size_t nval = ctx->h_nl_beta.size();
   if (columns) {
-    size_t tot = 0;
+    size_t tot = 0, off = 0;
     for (const auto& a : ctx->h_nl) tot += a.val.size();
     PWB_CHECK(ctx->h_nl.size() == (size_t)natom && tot == (size_t)np, PW_ENOTREADY,
               "analytic projector derivatives need the sets of pw_set_atoms");
-    for (int d = 0; d < 3; ++d) {
-      dcol[d].reserve(ctx->h_nl_beta.size());
-      for (const auto& a : ctx->h_nl)
-        for (const auto& v : a.val)
-          for (int g = 0; g < a.npts; ++g) dcol[d].push_back(v[4 * g + 1 + d]);
-      PWB_CHECK(dcol[d].size() == ctx->h_nl_beta.size(), PW_EINVAL, "projector sets changed since pw_set_atoms");
-    }
+    for (const auto& a : ctx->h_nl) off += a.val.size() * (size_t)a.npts;
+    PWB_CHECK(off == nval, PW_EINVAL, "projector sets changed since pw_set_atoms");
+    int rc = d_val4.alloc(std::max<size_t>(nval, 1) * 4 * 8);
+    if (rc) return rc;
+    off = 0;
+    for (const auto& a : ctx->h_nl)
+      for (const auto& v : a.val) {
+        if (a.npts)
+          PWB_CUDA(cudaMemcpyAsync((double*)d_val4.p + 4 * off, v.data(), (size_t)a.npts * 32, cudaMemcpyHostToDevice,
+                                   nullptr));
+        off += a.npts;
+      }
   }
   DevBuf d_idx, d_beta, d_pio, d_pbo, d_pnp, d_aoff, d_gl, d_cb, Qd, W, Wd, Qv, d_col;
   int rc;
-  if ((rc = upload(d_idx, ctx->h_nl_idx)) || (rc = upload(d_beta, ctx->h_nl_beta)) || (rc = upload(d_pio, ctx->h_pio)) ||
+  if ((rc = upload(d_idx, ctx->h_nl_idx)) || (rc = columns ? d_beta.alloc(std::max<size_t>(nval, 1) * 8) : upload(d_beta, ctx->h_nl_beta)) || (rc = upload(d_pio, ctx->h_pio)) ||
       (rc = upload(d_pbo, ctx->h_pbo)) || (rc = upload(d_pnp, ctx->h_pnp)) || (rc = upload(d_aoff, aoff)) ||
       (rc = upload(d_gl, gl)) || (rc = upload(d_cb, cb)) || (rc = Qd.alloc((size_t)np * nt * 8)) ||
       (rc = W.alloc((size_t)np * nb * 8)) || (rc = Wd.alloc((size_t)3 * np * nb * 8)))
     return rc;
   if ((rc = ensure_scratch(ctx, std::max(ctx->pair_cap, 1)))) return rc;
   const double* Q = (const double*)ctx->q.p;
+  const unsigned pick = (unsigned)std::min<size_t>(4096, (nval + 255) / 256 + 1);
+  if (columns) {
+    if ((rc = d_col.alloc(std::max<size_t>(nval, 1) * 8))) return rc;
+    k_pick_column<<<pick, 256>>>((const double*)d_val4.p, (long)nval, 0, (double*)d_beta.p);
+    ctx->launches += 1;
+  }
   if (ctx->nl_mode != PW_NL_DENSE || !ctx->have_nl) {
     // real-space projector mode keeps no coarse projector matrix: build one here
     if ((rc = Qv.alloc((size_t)np * nt * 8))) return rc;
@@ -234,7 +255,8 @@ static int nl_contract(pw_ctx* ctx, const double* psi, int ld, int nb, const std
   ctx->lib_launches += 1;
   for (int d = 0; d < 3; ++d) {
     if (columns) {
-      if ((rc = upload(d_col, dcol[d]))) return rc;
+      k_pick_column<<<pick, 256>>>((const double*)d_val4.p, (long)nval, 1 + d, (double*)d_col.p);
+      ctx->launches += 1;
       rc = run_build_q(ctx, (const int*)d_idx.p, (const double*)d_col.p, (const long*)d_pio.p, (const long*)d_pbo.p,
                        (const int*)d_pnp.p, np, nullptr, 0, Qd.p);
     } else {
