@@ -277,6 +277,13 @@ struct Launch {
   }
 };
 
+// whether the projector products run beside the FFT chain.  At every size: even
+// where a call is shorter than its launches, the products of one call then run
+// under the chain of the call before (Al4 20^3, 7 bands, calls back to back:
+// 38 us, in one stream 50 us)
+inline bool nl_beside_chain(const pw_ctx* c) {
+  return c->nl_mode == PW_NL_DENSE && c->have_nl && c->nproj > 0 && c->nl_overlap && !c->prof_on;
+}
 // a coarse-spectrum table from the host: [kz][ky][kx] into dst and [kz][kx][ky] into dst_t
 int upload_spectrum(pw_ctx* c, DevBuf& dst, DevBuf& dst_t, const double* src);
 

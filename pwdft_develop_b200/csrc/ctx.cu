@@ -210,7 +210,8 @@ int ensure_scratch(pw_ctx* c, int npair) {
 }
 
 // The band batch follows the calls: one launch per pass over all `npair` fields
-// where the batch fields fit in 1 GiB (Si64, 80 pairs: the five passes take
+// where the batch fields fit in 640 MiB (Si64 in FP64 just does; a new block costs
+// its first call about 7 ms per GB; Si64, 80 pairs: the five passes take
 // 400 us in one batch and 436 us in batches of 32, and the projector matrix
 // is read once, not three times).  It stays as it is once the caller has set it
 // and once a capture has recorded the buffers.  The passes then split the
@@ -224,7 +225,7 @@ int batch_pairs(pw_ctx* c, int npair, cudaStream_t st) {
   if (cs != cudaStreamCaptureStatusNone) c->mark_captured();
   if (npair > c->pair_cap && !c->batch_set && !c->captured) {
     const size_t per = (2 * (size_t)c->ntot + (size_t)c->nf[2] * (c->n[1] + 1) * (c->n[0] + 1)) * 2 * c->esz;
-    const int want = (int)std::min<size_t>(npair, ((size_t)1 << 30) / per), old = c->pair_cap;
+    const int want = (int)std::min<size_t>(npair, ((size_t)640 << 20) / per), old = c->pair_cap;
     if (want > old) {
       // other streams may still run passes on the present buffers; cudaFree waits for them
       c->pair_cap = 0;

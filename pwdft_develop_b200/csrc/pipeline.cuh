@@ -1421,14 +1421,13 @@ struct Plan {
     // dense projector mode: Q D Q^T psi depends on psi only, so its GEMMs run
     // on a second stream while the FFT chain runs (their first output goes to
     // the rows of out, which the last coarse pass then accumulates into after
-    // the join), for all bands of the call at once: Q is read once per call, not
-    // once per batch (Si216, 480 bands: Q is 1.6 GB).  The split bands take at
-    // most 1 GiB at a time.  With pw_profile on the products run batch by batch
+    // the join), in groups of their own that may be wider than a batch.  The split bands take at
+    // most 256 MiB at a time.  With pw_profile on the products run batch by batch
     // after the chain, so each kernel is timed alone
     const int nbnl = std::min(2 * npair, nband - band0);
     const bool dense_nl = c->nl_mode == PW_NL_DENSE && c->have_nl && c->nproj > 0 && nbnl > 0;
     cudaStream_t sn = nullptr;
-    if (dense_nl && c->nl_overlap && !c->prof_on) {
+    if (dense_nl && nl_beside_chain(c)) {
       if (!c->nl_st) PWB_CUDA(cudaStreamCreateWithFlags(&c->nl_st, cudaStreamNonBlocking));
       if (!c->nl_fork) PWB_CUDA(cudaEventCreateWithFlags(&c->nl_fork, cudaEventDisableTiming));
       if (!c->nl_join) PWB_CUDA(cudaEventCreateWithFlags(&c->nl_join, cudaEventDisableTiming));
@@ -1436,7 +1435,8 @@ struct Plan {
       if (band0 == 0) {
         PWB_CUDA(cudaEventRecord(c->nl_fork, st));
         PWB_CUDA(cudaStreamWaitEvent(sn, c->nl_fork, 0));
-        const int group = (int)std::max<long>(1, (1L << 30) / (4 * (long)c->ntot));
+        const int gmax = (int)std::max<long>(1, (256L << 20) / (4 * (long)c->ntot));
+        const int ngroup = (nband + gmax - 1) / gmax, group = (nband + ngroup - 1) / ngroup;
         for (int g0 = 0; g0 < nband; g0 += group)
           if ((rc = dense_apply(c, nl_set(c, filt), psi + (long)g0 * ld, ld, out + (long)g0 * ldo, ldo,
                                 std::min(group, nband - g0), sn, accumulate))) {

@@ -532,18 +532,24 @@ template <typename T, int NA, int NB> struct RFine {
   using RB = RegN<T, NB>;
   static constexpr int PM = RA::P > RB::P ? RA::P : RB::P;
   static constexpr int PS = NB + 1;
-  // threads: all 2 x 2 NA rows of one plane in one pass when one lane holds a
-  // row; several passes when two lanes do, where the row count divides them
-  // (30 pairs of 120 x 120: 192 threads 257 us, 256 threads 212 us; 32 of
-  // 144 x 144: 437 and 470 us)
-  static constexpr int TH = PM == 1 ? ceil32(4 * NA) : (4 * NA * RB::P % 256 >= 192 || 4 * NA * RB::P % 256 == 0 ? 256 : 192);
+  static constexpr size_t smem = sizeof(typename C2<T>::t) * (2 * NA * PS + (PM > 1 ? 2 * NA + 2 * NB : 0));
+  // threads: all 2 x 2 NA rows of a plane in one pass where that takes at most
+  // 320 lanes, else in the fewest equal passes of at most 320 (80 pairs, 192 / 256
+  // / 320 threads: FP32 72 1080 / 1178 / 1021 us, 60 - / 552 / 680, FP64 36 252 / 283
+  // / 242, 48 512 / 554 / 976); planes that leave room for one CTA only take 384
+  // (FP64 60, 40 pairs: 256 threads 897 us, 384 737)
+  static constexpr int LANES = 4 * NA * RB::P, NPASS = (LANES + 319) / 320;
+  static constexpr bool ALONE = 2 * (smem + 1024) > 227 * 1024;
+  static constexpr int TH = PM == 1 ? ceil32(4 * NA) : (ALONE ? 384 : (LANES / NPASS + 63) / 64 * 64);
   // FP32: only the two warps that share rows wait for one another (48: 239 ->
   // 234 us on 80 pairs of 96 x 96); FP64 stays in step (506, with pairs 551 us)
   static constexpr bool PAIR = sizeof(T) == 4 && TH % 64 == 0;
   static constexpr int CPP = TH / (2 * RA::P);   // columns (slots of B) per pass
   static constexpr int RPP = TH / (2 * RB::P);   // rows (fine points of A) per pass
-  static constexpr int MINB = reg_min_ctas<T, (RA::M > RB::M ? RA::M : RB::M)>(TH);
-  static constexpr size_t smem = sizeof(typename C2<T>::t) * (2 * NA * PS + (PM > 1 ? 2 * NA + 2 * NB : 0));
+  // one lane per row: 48 registers beside the data are enough (40: three CTAs
+  // instead of two, 164 -> 141 us on 80 pairs)
+  static constexpr int REGS = (RA::M > RB::M ? RA::M : RB::M) * 2 * (int)sizeof(T) / 4 + 48;
+  static constexpr int MINB = PM == 2 ? (ALONE ? 1 : 2) : (65536 / (REGS * TH) < 1 ? 1 : 65536 / (REGS * TH));
 };
 
 __device__ __forceinline__ void bar_pair(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
