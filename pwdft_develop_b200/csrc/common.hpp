@@ -47,7 +47,8 @@ struct PerDeviceOnce {
 };
 
 // Device buffer owned by a context.  With `keep` set, a block outgrown by a
-// later call goes there instead of being freed (a captured graph still reads it).
+// later call goes there instead of being freed (a captured graph may read it),
+// and its successor is at least half as large again.
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
@@ -217,14 +218,12 @@ struct pw_ctx {
   // scratch for the band-pair pipeline
   int pair_cap = 0;
   bool batch_set = false;          // pw_set_band_batch was called: the batch stays as set
-  bool captured = false;           // a stream capture has recorded this context's scratch
-  std::vector<void*> retired;      // outgrown blocks that a captured graph may still use; freed with the context
-  void mark_captured() {
-    if (captured) return;
-    captured = true;
-    for (pwb::DevBuf* b : {&s_ad, &s_k, &s_bc, &s_wp, &s_w, &s_wq, &s_psi_bf, &s_w_bf, &s_ws, &s_gx_bf, &s_gy_bf, &s_rot,
-                           &s_rot_x, &s_exx, &gsx_psir, &gsx_phir, &gsx_acc, &gsx_fields})
-      b->keep = &retired;
+  // blocks of the H*psi scratch outgrown by a later call: a graph captured before
+  // may still read them, so they live as long as the context (each block is at
+  // least half as large again as the one before: together at most twice the last)
+  std::vector<void*> retired;
+  void keep_scratch() {
+    for (pwb::DevBuf* b : {&s_ad, &s_k, &s_bc, &s_wp, &s_w, &s_wq, &s_psi_bf, &s_w_bf, &s_ws}) b->keep = &retired;
   }
   pwb::DevBuf s_ad, s_k, s_bc, s_wp, s_w;
   pwb::DevBuf s_host_in, s_host_out;   // device staging for the host-pointer entry points

@@ -20,6 +20,7 @@ void set_error(const std::string& msg) { g_err = msg; }
 int DevBuf::alloc(size_t nbytes) {
   if (nbytes <= bytes && p) return PW_OK;
   if (p && keep) {
+    nbytes = std::max(nbytes, bytes + bytes / 2);
     keep->push_back(p);
     p = nullptr;
     bytes = 0;
@@ -210,24 +211,21 @@ int ensure_scratch(pw_ctx* c, int npair) {
 }
 
 // The band batch follows the calls: one launch per pass over all `npair` fields
-// where the batch fields fit in 640 MiB (Si64 in FP64 just does; a new block costs
-// its first call about 7 ms per GB; Si64, 80 pairs: the five passes take
+// where the batch fields fit in 640 MiB (a new block costs
+// its first call about 7 ms per GB); Si64, 80 pairs: the five passes take
 // 400 us in one batch and 436 us in batches of 32, and the projector matrix
-// is read once, not three times).  It stays as it is once the caller has set it
-// and once a capture has recorded the buffers.  The passes then split the
-// bands evenly.
+// is read once, not three times).  It stays as it is once the caller has set it,
+// and in a call that is being captured.  The passes then split the bands evenly.
 int batch_pairs(pw_ctx* c, int npair, cudaStream_t st) {
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
-    cudaGetLastError();
-    cs = cudaStreamCaptureStatusActive;
-  }
-  if (cs != cudaStreamCaptureStatusNone) c->mark_captured();
-  if (npair > c->pair_cap && !c->batch_set && !c->captured) {
+  if (npair > c->pair_cap && !c->batch_set) {
     const size_t per = (2 * (size_t)c->ntot + (size_t)c->nf[2] * (c->n[1] + 1) * (c->n[0] + 1)) * 2 * c->esz;
     const int want = (int)std::min<size_t>(npair, ((size_t)640 << 20) / per), old = c->pair_cap;
-    if (want > old) {
-      // other streams may still run passes on the present buffers; cudaFree waits for them
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (want > old && cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+      cudaGetLastError();
+      cs = cudaStreamCaptureStatusActive;
+    }
+    if (want > old && cs == cudaStreamCaptureStatusNone) {
       c->pair_cap = 0;
       if (ensure_scratch(c, want)) {
         cudaGetLastError();
@@ -307,6 +305,7 @@ int pw_ctx_create(const double length[3], const int numGrid[3], const int numGri
   for (int s = 0; s < 6; ++s)
     if ((rc = upload_twiddles(c, s, lens[s]))) { delete c; return rc; }
   c->nl.cr = grid_chunk_rows(c->n, c->prec);
+  c->keep_scratch();
   if ((rc = ensure_scratch(c, 32))) { delete c; return rc; }
   {
     cublasHandle_t h;

@@ -33,7 +33,6 @@ int pw_graph_capture_hpsi(pw_ctx* ctx, const void* psi, int ld, void* hpsi, int 
   PWB_CUDA(cudaDeviceSynchronize());
   cudaStream_t st;
   PWB_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  ctx->mark_captured();
   const bool chk = ctx->check_errors;
   ctx->check_errors = false;   // the error-flag read synchronises; not allowed while capturing
   pw_graph* g = new pw_graph();
@@ -122,7 +121,6 @@ int pw_graph_capture_batch(int ncell, pw_ctx* const* ctxs, const void* const* ps
   std::vector<char> chk(ncell);
   for (int c = 0; c < ncell; ++c) {
     chk[c] = ctxs[c]->check_errors;
-    ctxs[c]->mark_captured();
     ctxs[c]->check_errors = false;
   }
   cudaStream_t st;

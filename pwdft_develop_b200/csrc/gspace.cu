@@ -345,6 +345,7 @@ int pw_ctx_create_gspace(const double length[3], const int numGrid[3], double ec
   const int lens[6] = {box[0], box[1], box[2], n0, n1, n2};
   for (int s = 0; s < 6; ++s)
     if ((rc = upload_twiddles(c, s, lens[s]))) { delete c; return rc; }
+  c->keep_scratch();
   if ((rc = ensure_scratch(c, 32))) { delete c; return rc; }
   {
     cublasHandle_t h;

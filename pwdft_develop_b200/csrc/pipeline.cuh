@@ -1422,7 +1422,7 @@ struct Plan {
     // on a second stream while the FFT chain runs (their first output goes to
     // the rows of out, which the last coarse pass then accumulates into after
     // the join), in groups of their own that may be wider than a batch.  The split bands take at
-    // most 256 MiB at a time.  With pw_profile on the products run batch by batch
+    // most 512 MiB at a time.  With pw_profile on the products run batch by batch
     // after the chain, so each kernel is timed alone
     const int nbnl = std::min(2 * npair, nband - band0);
     const bool dense_nl = c->nl_mode == PW_NL_DENSE && c->have_nl && c->nproj > 0 && nbnl > 0;
@@ -1435,7 +1435,7 @@ struct Plan {
       if (band0 == 0) {
         PWB_CUDA(cudaEventRecord(c->nl_fork, st));
         PWB_CUDA(cudaStreamWaitEvent(sn, c->nl_fork, 0));
-        const int gmax = (int)std::max<long>(1, (256L << 20) / (4 * (long)c->ntot));
+        const int gmax = (int)std::max<long>(1, (512L << 20) / (4 * (long)c->ntot));
         const int ngroup = (nband + gmax - 1) / gmax, group = (nband + ngroup - 1) / ngroup;
         for (int g0 = 0; g0 < nband; g0 += group)
           if ((rc = dense_apply(c, nl_set(c, filt), psi + (long)g0 * ld, ld, out + (long)g0 * ldo, ldo,
