@@ -407,7 +407,7 @@ typedef struct pw_tune_result {
   int cached;               /* 1: taken from the cache */
   double ms_default;        /* sweep time with the defaults */
   double ms_best;           /* sweep time with the chosen setting */
-  int fft_variant;          /* fused fine-plane transforms: 0 table twiddles, 1 second radix split, 2 (default) register twiddles */
+  int fft_variant;          /* H*psi transforms: 0 shared memory, 1 second radix split, 2 (default) registers */
 } pw_tune_result;
 /* Select the form of the fused fine-plane transforms directly (0: the first
  * radix decomposition N = n1 x n2 of each length with the inter-stage
@@ -561,7 +561,8 @@ PW_API int pw_teter_precond_noalloc(pw_ctx* ctx, const void* r, int ld, void* w,
                                     void* stream);
 
 /* Maximum number of bands processed per internal batch (sets scratch size).
- * Default 64. Scratch grows to hold ceil(nband_batch/2) band pairs. */
+ * Until this is called the batch follows the calls (scratch grows to the widest
+ * block, at most 640 MiB); afterwards it stays as set. */
 PW_API int pw_set_band_batch(pw_ctx* ctx, int nband_batch);
 
 /* ---- Restart files in the reference's binary layout ----

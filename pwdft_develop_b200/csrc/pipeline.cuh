@@ -13,6 +13,11 @@
 // the z-pencil kernels do that unfolding so the fine-plane kernels only see
 // plain zero padding.
 //
+// The default passes hold their transforms in registers (pipeline_reg.cuh: k_rfwd,
+// k_rzpad, k_rfloc, k_rzfold, k_rinv).  This file has the shared-memory form
+// of the same passes, used by the real-space projector mode, the density, the
+// projector build and fft_variant 0 / 1.
+//
 // Kernels (one launch each per band batch, all pairs in the grid):
 //   k_cxy_fwd    coarse plane: FFT x, FFT y                     psi -> A
 //   k_zpad       coarse z FFT, kinetic, unfold + pad, fine z IFFT  A -> K, B

@@ -1,6 +1,11 @@
 // H*psi, Teter and exchange passes with register-resident transforms
 // (regfft.cuh); included by pipeline.cuh.
 //
+// The shared-memory passes these replace wrote and read every element three
+// to nine times there and were bound by that; these are bound by HBM, the fine
+// plane by the FP32 / FP64 pipe and its barriers.  Times below: Si64, 80 pairs,
+// 48^3 / 96^3, before -> now.
+//
 // Layouts: spectra are [z][kx][ky] (ky fastest) so that both passes of a plane
 // load and store whole rows with one transform per lane and one exchange
 // through shared memory, and a z pencil needs none.  Slot fields are
@@ -54,7 +59,9 @@ template <typename T, int N0, int N1> struct RPlane {
 
 // Plane forward: values -> [z][kx][ky].  MODE 0: two real bands per field,
 // 1: complex bands, 2: exchange pairs psi_k (phi_ja + i phi_jb).  Bound by
-// memory: one read and one write of the field, one pass through shared memory.
+// memory: one read and one write of the field, one pass through shared memory
+// (FP32 62 -> 27 us, 5.2 TB/s; FP64 124 -> 49 us; exchange pairs 697 -> 248 us per
+// 1213 fields, bound by the three 4-byte reads per element from L2).
 struct RExx {
   int k0, ldp, j0, nphi, njp;
 };
@@ -139,7 +146,8 @@ k_rfwd(const T* __restrict__ psi, int ld, int nband, int band0, const T* __restr
   }
 }
 
-// Plane inverse: [z][kx][ky] -> values; CPLX as MODE 1 above
+// Plane inverse: [z][kx][ky] -> values; CPLX as MODE 1 above (FP32 54 -> 27 us, FP64
+// 120 -> 50 us)
 template <typename T, int N0, int N1, bool CPLX>
 __global__ void __launch_bounds__(RPlane<T, N0, N1>::TH, RPlane<T, N0, N1>::MINB)
 k_rinv(const VT<T>* __restrict__ D, T* __restrict__ out, int ldo, int nband, int band0, int accumulate, int n2) {
@@ -219,7 +227,9 @@ k_rinv(const VT<T>* __restrict__ D, T* __restrict__ out, int ldo, int nband, int
 
 // Exchange plane inverse: out_k (+)= sum_jp w_ja phi_ja Re + w_jb phi_jb Im of
 // the njp fields of band k0 + blockIdx.y; each lane owns its column's sums (in
-// shared memory, touched by no other lane)
+// shared memory, touched by no other lane: in registers they took 518-757 us for
+// 1024 fields against 433).  1213 fields: 1128 -> 463 us, bound by the two barriers
+// per field and 12 warps per SM
 template <typename T, int N0, int N1>
 __global__ void __launch_bounds__(RPlane<T, N0, N1>::TH, RPlane<T, N0, N1>::MINB)
 k_rexx_inv(const VT<T>* __restrict__ A, const T* __restrict__ phi, RExx ex, const T* __restrict__ wj,
@@ -298,7 +308,10 @@ template <typename T, int NZ> struct RPencil {
   static constexpr int MINBP = R::M * (int)sizeof(T) >= 144 ? 2 : reg_min_ctas<T, R::M>(THP);
 };
 
-// Teter / exchange kernel: FFT z, * table / N_c, IFFT z, in place
+// Teter / exchange kernel: FFT z, * table / N_c, IFFT z, in place: one read and one
+// write of the field (1213 fields of 48^3: 1107 -> 288 us, 7.4 TB/s).  The plane
+// size is a template argument: with a run-time stride the 48 addresses shared
+// by loads and stores stay live and spill (54 us instead of 21 for 80 fields).
 template <typename T, int N0, int N1, int NZ>
 __global__ void __launch_bounds__(RPencil<T, NZ>::TH, RPencil<T, NZ>::MINB)
 k_rzmul(VT<T>* __restrict__ A, const T* __restrict__ tab, T inv_nc) {
@@ -361,7 +374,10 @@ __device__ __forceinline__ void half_shift_all(typename C2<T>::t* v, int p, cons
 
 // z pencils up: coarse FFT z, kinetic term -> K, fine z values of the "+" (and,
 // on Nyquist rows and columns, "-") slots -> B.  The even fine planes are the
-// coarse values themselves, so the pencil costs two transforms of length NZ.
+// coarse values themselves, so the pencil costs two transforms of length NZ
+// (FP32 141 -> 60 us for 289 MB, FP64 285 -> 102 us; bound by the 96 strided stores
+// of each lane).  Slot rows stay N1 + 1 long: lanes run over row ends, and rows
+// padded to whole sectors were slower (72 us).
 template <typename T, int N0, int N1, int NZ>
 __global__ void __launch_bounds__(RPencil<T, NZ>::THP, RPencil<T, NZ>::MINBP)
 k_rzpad(const VT<T>* __restrict__ A, VT<T>* __restrict__ K, VT<T>* __restrict__ B, const T* __restrict__ ekin,
@@ -443,7 +459,8 @@ k_rzpad(const VT<T>* __restrict__ A, VT<T>* __restrict__ K, VT<T>* __restrict__ 
 
 // z pencils down: fold the fine z planes of the slots onto the coarse spectrum
 // (IP_f2c), add the kinetic term, inverse FFT z.  The even planes enter the
-// result as they are unless the cut-off mask needs their spectrum too.
+// result as they are unless the cut-off mask needs their spectrum too (FP32 133 ->
+// 53 us, with the mask 62 us; FP64 265 -> 95 us; bound by memory).
 template <typename T, int N0, int N1, int NZ, bool MASK>
 __global__ void __launch_bounds__(RPencil<T, NZ>::TH, RPencil<T, NZ>::MINB)
 k_rzfold(const VT<T>* __restrict__ C, const VT<T>* __restrict__ K, VT<T>* __restrict__ D,
@@ -525,7 +542,12 @@ k_rzfold(const VT<T>* __restrict__ C, const VT<T>* __restrict__ K, VT<T>* __rest
 // are separate tasks of the two halves of the CTA; on the way back the halves
 // swap one half of their outputs through shared memory and add.
 // Shared memory per plane: 2 NA (NB + 1) elements written and read about three
-// times, against nine in k_floc2.
+// times, against nine in k_floc2.  FP32 280 -> 234 us, FP64 617 -> 508 us, 144 x 144
+// planes (80 pairs, FP32) 1326 -> 1021 us: the FP32 pipe is busy 48 % of the time
+// (12 warps of 158 registers; barriers are the first stall, the instruction
+// cache the next: the four transforms are about 50 KB of code).  Slower: packed
+// two-value FP32 instructions (244-274 us: register moves), one shared copy of the
+// transform in a loop (255-272), 96 or 128 threads (263, 260), 128 registers (272).
 // ---------------------------------------------------------------------------
 template <typename T, int NA, int NB> struct RFine {
   using RA = RegN<T, NA>;

@@ -2,7 +2,9 @@
 //
 // A transform of length N lives in the registers of P lanes, M = N / P
 // elements each: one lane up to 48 elements in FP32 (96 registers of data)
-// and 24 (or 30) in FP64, two lanes above.  Nothing goes through shared memory inside
+// and 24 (or 30) in FP64, two lanes above (80 fields of z pencils, forward, table,
+// inverse: 60 in one lane 61 us, in two 53; 72 119 and 85; one lane of 48 in FP64
+// would need 192 registers of data).  Nothing goes through shared memory inside
 // a transform; the two-lane form exchanges M / 2 elements by shuffles for its
 // last (first) radix-2 stage.
 //
