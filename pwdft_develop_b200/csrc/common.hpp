@@ -47,13 +47,16 @@ struct PerDeviceOnce {
 };
 
 // Device buffer owned by a context.  With `keep` set, a block outgrown by a
-// later call goes there instead of being freed (a captured graph may read it),
-// and its successor is at least half as large again.
+// later call goes there instead of being freed (a captured graph may read it);
+// the new block is allocated first, and a failure leaves the old one in use.  grow() asks for half as much again as
+// the block it replaces, so that many small steps keep little (alloc() if that
+// is refused).
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
   std::vector<void*>* keep = nullptr;
   int alloc(size_t nbytes);
+  int grow(size_t nbytes);
   void release();
   ~DevBuf() { release(); }
   DevBuf() = default;
@@ -217,10 +220,9 @@ struct pw_ctx {
   std::vector<cudaEvent_t> ev_pool;
   // scratch for the band-pair pipeline
   int pair_cap = 0;
-  bool batch_set = false;          // pw_set_band_batch was called: the batch stays as set
+  bool batch_set = false;          // pw_set_band_batch was called (or a growth refused): the batch stays
   // blocks of the H*psi scratch outgrown by a later call: a graph captured before
-  // may still read them, so they live as long as the context (each block is at
-  // least half as large again as the one before: together at most twice the last)
+  // may still read them, so they live as long as the context
   std::vector<void*> retired;
   void keep_scratch() {
     for (pwb::DevBuf* b : {&s_ad, &s_k, &s_bc, &s_wp, &s_w, &s_wq, &s_psi_bf, &s_w_bf, &s_ws}) b->keep = &retired;

@@ -17,31 +17,6 @@ namespace pwb {
 static thread_local std::string g_err;
 void set_error(const std::string& msg) { g_err = msg; }
 
-int DevBuf::alloc(size_t nbytes) {
-  if (nbytes <= bytes && p) return PW_OK;
-  if (p && keep) {
-    nbytes = std::max(nbytes, bytes + bytes / 2);
-    keep->push_back(p);
-    p = nullptr;
-    bytes = 0;
-  }
-  release();
-  if (nbytes == 0) return PW_OK;
-  cudaError_t e = cudaMalloc(&p, nbytes);
-  if (e != cudaSuccess) {
-    p = nullptr;
-    set_error(std::string("cudaMalloc failed: ") + cudaGetErrorString(e));
-    return PW_ENOMEM;
-  }
-  bytes = nbytes;
-  return PW_OK;
-}
-void DevBuf::release() {
-  if (p) cudaFree(p);
-  p = nullptr;
-  bytes = 0;
-}
-
 // defined in hpsi.cu
 int grid_chunk_rows(const int n[3], int prec);
 int run_hpsi(pw_ctx* c, const void* psi, int ld, void* out, int ldo, int nband, int band0, int npair, int acc,
@@ -151,6 +126,7 @@ int wfn_filter_pass(pw_ctx* c, void* X, int ld, int nb, cudaStream_t st) {
   c->teter_tab = c->wmask.p;
   int rc = PW_OK;
   const int cap = c->pair_cap;
+  if (cap < 1) rc = PW_ENOMEM;
   for (int b0 = 0; b0 < nb && !rc; b0 += 2 * cap) {
     const int npair = std::min(cap, (nb - b0 + 1) / 2);
     rc = run_teter(c, X, ld, X, ld, nb, b0, npair, 0, st);
@@ -194,20 +170,38 @@ int prepare_wfn_filter(pw_ctx* c) {
   return PW_OK;
 }
 
-int ensure_scratch(pw_ctx* c, int npair) {
-  if (npair <= c->pair_cap && c->s_ad.p) return PW_OK;
+// room for npair pairs in every block of the H*psi scratch; a failure leaves the
+// blocks that were there (or grew already)
+static int alloc_scratch(pw_ctx* c, int npair) {
   const size_t cs = 2 * c->esz;   // complex element
   const size_t nb = (size_t)c->nf[2] * (c->n[1] + 1) * (c->n[0] + 1);
   int rc;
+  // the largest first: a growth that does not fit then takes nothing
+  if ((rc = c->s_bc.alloc((size_t)npair * nb * cs))) return rc;
   if ((rc = c->s_ad.alloc((size_t)npair * c->ntot * cs))) return rc;
   if ((rc = c->s_k.alloc((size_t)npair * c->ntot * cs))) return rc;
-  if ((rc = c->s_bc.alloc((size_t)npair * nb * cs))) return rc;
   const size_t nslot = std::max(1, c->nl.nslot), nat = std::max(1, c->nl.natom), np = std::max(1, c->nl.npmax);
   if ((rc = c->s_wp.alloc((size_t)npair * nslot * np * cs))) return rc;
   if ((rc = c->s_w.alloc((size_t)npair * nat * np * cs))) return rc;
-  if ((rc = c->s_wq.alloc((size_t)std::max(1, c->nproj) * 2 * npair * c->esz))) return rc;
-  c->pair_cap = npair;
-  return PW_OK;
+  return c->s_wq.grow((size_t)std::max(1, c->nproj) * 2 * npair * c->esz);
+}
+
+// at least npair pairs; a failure leaves the batch as it was
+int ensure_scratch(pw_ctx* c, int npair) {
+  if (npair <= c->pair_cap && c->s_ad.p) return PW_OK;
+  const int rc = alloc_scratch(c, npair);
+  if (!rc) c->pair_cap = npair;
+  return rc;
+}
+
+// after the projector tables changed: the batch again, halved until it fits
+int refit_scratch(pw_ctx* c) {
+  int rc = PW_ENOMEM;
+  for (int np = std::max(c->pair_cap, 1); np >= 1 && rc; np /= 2) {
+    rc = alloc_scratch(c, np);
+    c->pair_cap = rc ? 0 : np;
+  }
+  return rc;
 }
 
 // The band batch follows the calls: one launch per pass over all `npair` fields
@@ -215,28 +209,22 @@ int ensure_scratch(pw_ctx* c, int npair) {
 // its first call about 7 ms per GB); Si64, 80 pairs: the five passes take
 // 400 us in one batch and 436 us in batches of 32, and the projector matrix
 // is read once, not three times).  It stays as it is once the caller has set it,
-// and in a call that is being captured.  The passes then split the bands evenly.
+// once a growth was refused, and in a call that is being captured.  The passes
+// then split the bands evenly.
 int batch_pairs(pw_ctx* c, int npair, cudaStream_t st) {
   if (npair > c->pair_cap && !c->batch_set) {
     const size_t per = (2 * (size_t)c->ntot + (size_t)c->nf[2] * (c->n[1] + 1) * (c->n[0] + 1)) * 2 * c->esz;
-    const int want = (int)std::min<size_t>(npair, ((size_t)640 << 20) / per), old = c->pair_cap;
+    const int want = (int)std::min<size_t>(npair, ((size_t)640 << 20) / per);
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (want > old && cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+    if (want > c->pair_cap && cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
       cudaGetLastError();
       cs = cudaStreamCaptureStatusActive;
     }
-    if (want > old && cs == cudaStreamCaptureStatusNone) {
-      c->pair_cap = 0;
-      if (ensure_scratch(c, want)) {
-        cudaGetLastError();
-        c->pair_cap = 0;
-        if (ensure_scratch(c, old)) return 0;
-        c->batch_set = true;     // no room: keep the old batch
-      }
-    }
+    if (want > c->pair_cap && cs == cudaStreamCaptureStatusNone && ensure_scratch(c, want)) c->batch_set = true;
   }
-  const int nb = (npair + c->pair_cap - 1) / std::max(1, c->pair_cap);
-  return c->pair_cap < 1 ? 0 : (npair + nb - 1) / std::max(1, nb);
+  if (c->pair_cap < 1) return 0;
+  const int nb = (npair + c->pair_cap - 1) / c->pair_cap;
+  return (npair + nb - 1) / std::max(1, nb);
 }
 
 }  // namespace pwb
@@ -402,9 +390,12 @@ int pw_set_check_errors(pw_ctx* ctx, int enable) {
 int pw_set_band_batch(pw_ctx* ctx, int nband_batch) {
   PWB_CHECK(ctx && nband_batch > 0, PW_EINVAL, "bad band batch");
   PWB_CUDA(cudaSetDevice(ctx->device));
-  ctx->pair_cap = 0;
+  const int npair = (nband_batch + 1) / 2;
+  const int rc = alloc_scratch(ctx, npair);
+  if (rc) return rc;      // the batch stays as it was
+  ctx->pair_cap = npair;
   ctx->batch_set = true;
-  return ensure_scratch(ctx, (nband_batch + 1) / 2);
+  return PW_OK;
 }
 
 int pw_set_nonlocal(pw_ctx* ctx, int natom, const int* atom_npts, const int* atom_nproj, const int* idx,
@@ -485,9 +476,7 @@ int pw_set_nonlocal(pw_ctx* ctx, int natom, const int* atom_npts, const int* ato
       PWB_CUDA(cudaMemcpy(d_pnp.p, pnp.data(), nproj * 4, cudaMemcpyHostToDevice));
       if ((rc = ctx->q.alloc((size_t)nproj * ctx->ntot * ctx->esz))) return rc;
       if ((rc = upload_real(ctx, ctx->qd, qd.data(), nproj))) return rc;
-      const int cap = std::max(ctx->pair_cap, 1);
-      ctx->pair_cap = 0;
-      if ((rc = ensure_scratch(ctx, cap))) return rc;
+      if ((rc = refit_scratch(ctx))) return rc;
       rc = run_build_q(ctx, (const int*)d_idx.p, (const double*)d_beta.p, (const long*)d_pio.p,
                        (const long*)d_pbo.p, (const int*)d_pnp.p, nproj, nullptr);
       if (rc) return rc;
@@ -582,9 +571,7 @@ int pw_set_nonlocal(pw_ctx* ctx, int natom, const int* atom_npts, const int* ato
   nl.ntile = ntile;
   nl.nchunk = nchunk;
   ctx->have_nl = true;
-  const int cap = std::max(ctx->pair_cap, 1);
-  ctx->pair_cap = 0;
-  return ensure_scratch(ctx, cap);
+  return refit_scratch(ctx);
 }
 
 int pw_hpsi(pw_ctx* ctx, const void* psi, int ld, void* hpsi, int ldh, int nband, int accumulate, void* stream) {

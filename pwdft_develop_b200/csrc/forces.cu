@@ -374,6 +374,7 @@ int pw_band_energy_backward(pw_ctx* ctx, const void* psi, int ld, int nband, con
       for (int b = 0; b < nband; ++b) h[b] = w[b] * (double)ctx->ntot / (double)ctx->ntotf;
       PWB_CUDA(cudaMemcpy(wv.p, h.data(), h.size() * 8, cudaMemcpyHostToDevice));
       const int cap = ctx->pair_cap;
+      PWB_CHECK(cap > 0, PW_ENOMEM, "no device scratch");
       for (int b0 = 0; b0 < nband; b0 += 2 * cap) {
         const int npair = std::min(cap, (nband - b0 + 1) / 2);
         if ((rc = run_density(ctx, psi, ld, nband, b0, npair, (const double*)wv.p, dE_dV_dev, nullptr))) return rc;

@@ -651,7 +651,7 @@ int gemm_tn_reduce(const SplitOperand& A, const SplitOperand& B, int K, int nter
   nsplit = std::max(nsplit, (K + KCHUNK_MAX - 1) / KCHUNK_MAX);
   int kchunk = ((K + nsplit - 1) / nsplit + GK - 1) / GK * GK;
   nsplit = (K + kchunk - 1) / kchunk;
-  int rc = ws.alloc((size_t)nbatch * nsplit * M * N * sizeof(float));
+  int rc = ws.grow((size_t)nbatch * nsplit * M * N * sizeof(float));
   if (rc) return rc;
   GemmArgs g{};
   g.M = M; g.N = N; g.K = K; g.kchunk = kchunk; g.nterms = nterms; g.epi = 0;

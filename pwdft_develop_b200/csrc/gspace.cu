@@ -27,6 +27,7 @@ namespace pwb {
 int upload_real(pw_ctx* c, DevBuf& dst, const double* src, size_t n);
 int upload_twiddles(pw_ctx* c, int slot, int n);
 int ensure_scratch(pw_ctx* c, int npair);
+int refit_scratch(pw_ctx* c);
 int install_dense_q(pw_ctx* ctx, int nproj);
 
 namespace {
@@ -395,9 +396,7 @@ int pw_gs_set_projectors(pw_ctx* ctx, int nproj, const double* vnlc, const doubl
   ctx->h_nl_beta.assign(vnlc, vnlc + (size_t)nproj * ctx->ntot);
   ctx->h_pgamma.assign(wgt, wgt + nproj);
   ctx->have_nl = true;
-  const int cap = std::max(ctx->pair_cap, 1);
-  ctx->pair_cap = 0;
-  return ensure_scratch(ctx, cap);
+  return refit_scratch(ctx);
 }
 
 int pw_gs_get_projectors(const pw_ctx* ctx, int* nproj, double* vnlc, double* wgt) {

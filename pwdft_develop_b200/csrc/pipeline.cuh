@@ -1608,7 +1608,7 @@ struct Plan {
     if (cublasSetStream(h, st) != CUBLAS_STATUS_SUCCESS) { set_error("cublasSetStream failed"); return PW_ECUDA; }
     const int np = ds.np, nt = (int)c->ntot;
     int rc;
-    if ((rc = c->s_wq.alloc((size_t)np * nb * sizeof(T)))) return rc;
+    if ((rc = c->s_wq.grow((size_t)np * nb * sizeof(T)))) return rc;
     T* W = reinterpret_cast<T*>(c->s_wq.p);
     const T* Q = reinterpret_cast<const T*>(ds.q);
     const T one = 1, zero = 0;
@@ -1662,8 +1662,8 @@ struct Plan {
     // maps cover K = nt, so the pad is never read
     const long ntp = (nt + 7) / 8 * 8;
     int rc;
-    if ((rc = c->s_psi_bf.alloc((size_t)2 * nb * ntp * 2))) return rc;
-    if ((rc = c->s_w_bf.alloc((size_t)2 * nb * npp * 2))) return rc;
+    if ((rc = c->s_psi_bf.grow((size_t)2 * nb * ntp * 2))) return rc;
+    if ((rc = c->s_w_bf.grow((size_t)2 * nb * npp * 2))) return rc;
     char* pb = (char*)c->s_psi_bf.p;
     char* wb = (char*)c->s_w_bf.p;
     { Launch L_(c, st, KK_MISC);
@@ -1768,8 +1768,8 @@ struct Plan {
     int rc;
     const size_t nf = (size_t)nk * nb;
     const long kstep = (long)(kq_bf_bytes(c) / 2);
-    if ((rc = c->s_psi_bf.alloc(2 * nf * nt2 * 2))) return rc;
-    if ((rc = c->s_w_bf.alloc(2 * nf * np2 * 2))) return rc;
+    if ((rc = c->s_psi_bf.grow(2 * nf * nt2 * 2))) return rc;
+    if ((rc = c->s_w_bf.grow(2 * nf * np2 * 2))) return rc;
     char* pb = (char*)c->s_psi_bf.p;
     char* wb = (char*)c->s_w_bf.p;
     { Launch L_(c, st, KK_MISC);
@@ -1804,7 +1804,7 @@ struct Plan {
     cublasHandle_t h = (cublasHandle_t)c->blas;
     if (cublasSetStream(h, st) != CUBLAS_STATUS_SUCCESS) { set_error("cublasSetStream failed"); return PW_ECUDA; }
     const int np = c->nproj, nt = (int)c->ntot;
-    if ((rc = c->s_wq.alloc((size_t)np * nb * sizeof(V)))) return rc;
+    if ((rc = c->s_wq.grow((size_t)np * nb * sizeof(V)))) return rc;
     V* W = reinterpret_cast<V*>(c->s_wq.p);
     cublasStatus_t r;
     { Launch L_(c, st, KK_LIBGEMM);

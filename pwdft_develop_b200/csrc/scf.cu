@@ -1670,6 +1670,7 @@ int pw_scf_run(pw_ctx* ctx, const pw_scf_params* p, pw_scf_result* r, double* ei
       PWB_CUDA(cudaMemcpy(S.wocc.p, wv.data(), wv.size() * 8, cudaMemcpyHostToDevice));
       PWB_CUDA(cudaMemset(ro, 0, nf * 8));
       const int cap = sv.c->pair_cap;
+      PWB_CHECK(cap > 0, PW_ENOMEM, "no device scratch");
       for (int b0 = 0; b0 < nb; b0 += 2 * cap) {
         const int npair = std::min(cap, (nb - b0 + 1) / 2);
         if ((rc = run_density(sv.c, sv.X.p, (int)nt, nb, b0, npair, (const double*)S.wocc.p, ro, nullptr))) return rc;
@@ -2140,6 +2141,7 @@ int pw_density(pw_ctx* ctx, const void* psi, int ld, int nband, const double* oc
   PWB_CUDA(cudaMemcpy(wv.p, h.data(), h.size() * 8, cudaMemcpyHostToDevice));
   PWB_CUDA(cudaMemset(rho_dev, 0, ctx->ntotf * 8));
   const int cap = ctx->pair_cap;
+  PWB_CHECK(cap > 0, PW_ENOMEM, "no device scratch");
   for (int b0 = 0; b0 < nband; b0 += 2 * cap) {
     const int npair = std::min(cap, (nband - b0 + 1) / 2);
     if ((rc = run_density(ctx, psi, ld, nband, b0, npair, (const double*)wv.p, rho_dev, nullptr))) return rc;

@@ -81,3 +81,28 @@ def test_kpoint_batches(prec, batch):
         ref = c.hpsi_k(x[i].contiguous())
         err = (got[i] - ref).abs().max() / ref.abs().max()
         assert err <= (1e-5 if prec == "f32" else 1e-13), (i, float(err))
+
+
+@pytest.mark.parametrize("prec", ["f64"])
+def test_a_refused_growth_leaves_the_batch(prec):
+    """No room for a larger batch: the call runs in the batch that is there."""
+    import torch
+    from pwdft_develop_b200._lib import PwError
+    c = _ctx(prec)
+    x = _rand(c, 900)
+    out = torch.empty_like(x)
+    ref = torch.cat([c.hpsi(x[i:i + 30]) for i in range(0, 900, 30)])
+    with pytest.raises(PwError):
+        c.set_band_batch(2000000000)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (40 << 20), dtype=torch.uint8, device="cuda")
+    for _ in range(3):
+        out.zero_()
+        c.hpsi(x, out=out)
+        torch.cuda.synchronize()
+    del fill
+    torch.cuda.empty_cache()
+    # other widths of the projector products: equal to rounding
+    assert (out - ref).abs().max() <= (1e-5 if prec == "f32" else 1e-13) * ref.abs().max()
+    assert (c.hpsi(x) - ref).abs().max() <= (1e-5 if prec == "f32" else 1e-13) * ref.abs().max()
