@@ -48,7 +48,8 @@ struct PerDeviceOnce {
 
 // Device buffer owned by a context.  With `keep` set, a block outgrown by a
 // later call goes there instead of being freed (a captured graph may read it);
-// the new block is allocated first, and a failure leaves the old one in use.  grow() asks for half as much again as
+// the new block is allocated first, also while a stream is being captured, and
+// a failure leaves the old one in use.  grow() asks for half as much again as
 // the block it replaces, so that many small steps keep little (alloc() if that
 // is refused).
 struct DevBuf {

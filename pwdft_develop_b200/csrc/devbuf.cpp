@@ -7,6 +7,15 @@ namespace pwb {
 
 namespace {
 
+// cudaMalloc is forbidden while this thread, or (global mode) any thread,
+// captures a stream, unless the calling thread works in relaxed mode; the
+// allocation itself does not become part of the graph
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 int device_alloc(void** p, size_t nbytes) {
   const cudaError_t e = cudaMalloc(p, nbytes);
   if (e == cudaSuccess) return PW_OK;
@@ -28,6 +37,7 @@ int DevBuf::alloc(size_t nbytes) {
     return rc;
   }
   if (nbytes == 0) return PW_OK;
+  RelaxedCapture guard;
   void* q = nullptr;
   const int rc = device_alloc(&q, nbytes);
   if (rc) return rc;      // the block in use stays in use

@@ -1426,9 +1426,8 @@ struct Plan {
     // dense projector mode: Q D Q^T psi depends on psi only, so its GEMMs run
     // on a second stream while the FFT chain runs (their first output goes to
     // the rows of out, which the last coarse pass then accumulates into after
-    // the join), in groups of their own that may be wider than a batch.  The split bands take at
-    // most 512 MiB at a time.  With pw_profile on the products run batch by batch
-    // after the chain, so each kernel is timed alone
+    // the join), all bands of the call together (dense_call).  With pw_profile on
+    // the products run batch by batch after the chain, so each kernel is timed alone
     const int nbnl = std::min(2 * npair, nband - band0);
     const bool dense_nl = c->nl_mode == PW_NL_DENSE && c->have_nl && c->nproj > 0 && nbnl > 0;
     cudaStream_t sn = nullptr;
@@ -1440,15 +1439,12 @@ struct Plan {
       if (band0 == 0) {
         PWB_CUDA(cudaEventRecord(c->nl_fork, st));
         PWB_CUDA(cudaStreamWaitEvent(sn, c->nl_fork, 0));
-        const int gmax = (int)std::max<long>(1, (512L << 20) / (4 * (long)c->ntot));
-        const int ngroup = (nband + gmax - 1) / gmax, group = (nband + ngroup - 1) / ngroup;
-        for (int g0 = 0; g0 < nband; g0 += group)
-          if ((rc = dense_apply(c, nl_set(c, filt), psi + (long)g0 * ld, ld, out + (long)g0 * ldo, ldo,
-                                std::min(group, nband - g0), sn, accumulate))) {
-            cudaStreamWaitEvent(st, c->nl_fork, 0);
-            return rc;
-          }
+        rc = dense_call(c, nl_set(c, filt), psi, ld, out, ldo, nband, sn, accumulate);
         PWB_CUDA(cudaEventRecord(c->nl_join, sn));
+        if (rc) {
+          cudaStreamWaitEvent(st, c->nl_join, 0);
+          return rc;
+        }
       }
     }
     if (reg(c) && c->nl_mode == PW_NL_DENSE) {
@@ -1625,6 +1621,27 @@ struct Plan {
     PWB_CUDA(cudaGetLastError());
     return PW_OK;
     }
+  }
+
+  // dense_apply over all bands of a call, in even groups whose split bands take at
+  // most 512 MiB, halved while their operands find no room (PW_ENOMEM comes
+  // before anything is written to out)
+  static int dense_call(pw_ctx* c, const DenseSet& ds, const T* psi, int ld, T* out, int ldo, int nb, cudaStream_t st,
+                        int acc = 1) {
+    const int gmax = (int)std::max<long>(1, (512L << 20) / (4 * (long)c->ntot));
+    const int ngroup = (nb + gmax - 1) / gmax;
+    int group = (nb + ngroup - 1) / std::max(1, ngroup);
+    for (int g0 = 0; g0 < nb;) {
+      const int n = std::min(group, nb - g0);
+      const int rc = dense_apply(c, ds, psi + (long)g0 * ld, ld, out + (long)g0 * ldo, ldo, n, st, acc);
+      if (rc == PW_ENOMEM && n > 1) {
+        group = (n + 1) / 2;
+        continue;
+      }
+      if (rc) return rc;
+      g0 += n;
+    }
+    return PW_OK;
   }
 
   // rho += sum over the batch's bands of w_b |psi_b,fine|^2 (unnormalised)

@@ -83,7 +83,7 @@ def test_kpoint_batches(prec, batch):
         assert err <= (1e-5 if prec == "f32" else 1e-13), (i, float(err))
 
 
-@pytest.mark.parametrize("prec", ["f64"])
+@pytest.mark.parametrize("prec", ["f32", "f64"])
 def test_a_refused_growth_leaves_the_batch(prec):
     """No room for a larger batch: the call runs in the batch that is there."""
     import torch
@@ -106,3 +106,39 @@ def test_a_refused_growth_leaves_the_batch(prec):
     # other widths of the projector products: equal to rounding
     assert (out - ref).abs().max() <= (1e-5 if prec == "f32" else 1e-13) * ref.abs().max()
     assert (c.hpsi(x) - ref).abs().max() <= (1e-5 if prec == "f32" else 1e-13) * ref.abs().max()
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+def test_capture_of_a_call_wider_than_any_before(prec):
+    """Recorded on a capturing stream, a block wider than the scratch runs in the
+    batch that is there and its projector products still find their operands."""
+    import torch
+    c = _ctx(prec)
+    c.hpsi(_rand(c, 6))
+    x = _rand(c, 203, seed=8)
+    out = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        c.hpsi(x, out=out)
+    x.copy_(_rand(c, 203, seed=9))
+    g.replay()
+    torch.cuda.synchronize()
+    ref = c.hpsi(x)
+    assert (out - ref).abs().max() <= (1e-5 if prec == "f32" else 1e-13) * ref.abs().max()
+
+
+def test_projector_products_of_more_than_one_group():
+    """363 bands of 72^3 are two groups of split bands and seven batches; against
+    narrow calls, whose products have other tiles and partitions (FP32 bar)."""
+    import torch
+    c = _ctx("f32", n=(72, 72, 72))
+    nb = 363
+    assert nb * 4 * c.ntot > 512 << 20
+    x = _rand(c, nb)
+    ref = torch.cat([c.hpsi(x[i:i + 33]) for i in range(0, nb, 33)])
+    top = ref.abs().max()
+    assert (c.hpsi(x) - ref).abs().max() <= 1e-5 * top
+    base = torch.randn_like(x[:1]).expand(nb, -1).contiguous()
+    got = c.hpsi(x, out=base.clone(), accumulate=True)
+    assert (got - (base + ref)).abs().max() <= 1e-5 * top
