@@ -58,6 +58,7 @@ struct DevBuf {
   std::vector<void*>* keep = nullptr;
   int alloc(size_t nbytes);
   int grow(size_t nbytes);
+  void drop();               // given back: freed, or kept for captured graphs
   void release();
   ~DevBuf() { release(); }
   DevBuf() = default;
@@ -227,6 +228,18 @@ struct pw_ctx {
   std::vector<void*> retired;
   void keep_scratch() {
     for (pwb::DevBuf* b : {&s_ad, &s_k, &s_bc, &s_wp, &s_w, &s_wq, &s_psi_bf, &s_w_bf, &s_ws}) b->keep = &retired;
+  }
+  // the exchange workspaces (1 GiB and more) are freed when outgrown until an
+  // exchange is recorded by a capturing stream
+  void keep_exx_scratch(cudaStream_t st) {
+    if (s_exx.keep) return;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+      cudaGetLastError();
+      cs = cudaStreamCaptureStatusActive;
+    }
+    if (cs == cudaStreamCaptureStatusNone) return;
+    for (pwb::DevBuf* b : {&s_exx, &gsx_psir, &gsx_phir, &gsx_acc, &gsx_fields}) b->keep = &retired;
   }
   pwb::DevBuf s_ad, s_k, s_bc, s_wp, s_w;
   pwb::DevBuf s_host_in, s_host_out;   // device staging for the host-pointer entry points

@@ -53,6 +53,14 @@ int DevBuf::grow(size_t nbytes) {
   return alloc(nbytes);
 }
 
+void DevBuf::drop() {
+  if (p && keep) {
+    keep->push_back(p);
+    p = nullptr;
+  }
+  release();
+}
+
 void DevBuf::release() {
   if (p) cudaFree(p);
   p = nullptr;

@@ -185,7 +185,7 @@ int pw_exx_set_phi(pw_ctx* ctx, const void* psi, int ld, int nphi, const double*
 int pw_exx_set_scratch(pw_ctx* ctx, size_t bytes) {
   PWB_CHECK(ctx && bytes > 0, PW_EINVAL, "bad arguments");
   ctx->exx_scratch_bytes = bytes;
-  ctx->s_exx.release();
+  ctx->s_exx.drop();
   return PW_OK;
 }
 

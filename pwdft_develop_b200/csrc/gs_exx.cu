@@ -223,6 +223,7 @@ int gs_exx_apply_t(pw_ctx* c, const T* psi, int ld, int nb, T* out, int ldo, int
   int rc;
   const size_t phib = (size_t)nphi * n3 * sizeof(T);
   if (phir.bytes < phib) c->gsx_phi_ready = false;
+  c->keep_exx_scratch(st);
   if ((rc = psir.alloc((size_t)nb * n3 * sizeof(T))) || (rc = phir.alloc(phib)) ||
       (rc = acc.alloc((size_t)nb * n3 * sizeof(T))) ||
       (rc = F.alloc((size_t)std::max<long>((long)kb * njp, pcap) * n3 * sizeof(V))))

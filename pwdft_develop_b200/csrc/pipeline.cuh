@@ -1568,6 +1568,7 @@ struct Plan {
     const long cap = std::max<long>(1, (long)(c->exx_scratch_bytes / ((size_t)nt * sizeof(V))));
     const int jc = (int)std::min<long>(njp, std::max<long>(1, cap / nb));
     const int kc = (int)std::max<long>(1, std::min<long>(nb, cap / jc));
+    c->keep_exx_scratch(st);
     if ((rc = c->s_exx.alloc((size_t)kc * jc * nt * sizeof(V)))) return rc;
     V* A = reinterpret_cast<V*>(c->s_exx.p);
     const T* phi = reinterpret_cast<const T*>(c->exx_phi.p);

@@ -76,6 +76,21 @@ int main() {
     CHECK(b.bytes < 1500000);
   }
   for (void* p : kept) cudaFree(p);
+  kept.clear();
+  {
+    // a block that a capture may have recorded is neither freed by a growth nor given back
+    pwb::DevBuf b;
+    g_limit = 1000;
+    CHECK(b.alloc(60) == PW_OK);
+    void* p = b.p;
+    b.keep = &kept;
+    CHECK(b.alloc(90) == PW_OK && kept.size() == 1 && kept[0] == p && g_live.count(p));
+    void* q = b.p;
+    b.drop();
+    CHECK(!b.p && !b.bytes && kept.size() == 2 && g_live.count(q) && g_used == 150);
+    CHECK(b.alloc(30) == PW_OK && b.bytes == 30);
+  }
+  for (void* p : kept) cudaFree(p);
   {
     // without `keep` the old block is freed before the new one is asked for
     pwb::DevBuf b;

@@ -142,3 +142,39 @@ def test_projector_products_of_more_than_one_group():
     base = torch.randn_like(x[:1]).expand(nb, -1).contiguous()
     got = c.hpsi(x, out=base.clone(), accumulate=True)
     assert (got - (base + ref)).abs().max() <= 1e-5 * top
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("mode", ["planes", "sphere"])
+def test_a_captured_exchange_outlives_larger_ones(mode, prec):
+    """H*psi with the full exchange, recorded; then a wider exchange and another
+    scratch limit: the recorded workspaces are still the graph's."""
+    import torch
+    if mode == "planes":
+        c = _ctx(prec)
+    else:
+        from oracle import pw
+        from pwdft_develop_b200 import Context
+        L, z, pos = pw.make_crystal("Si", (1, 1, 1), A, 0.02, 77)
+        c = Context.gspace(L, (32, 32, 32), 6.0, precision=prec)
+        c.set_atoms([z] * len(pos), pos)
+        c.set_vtot(np.random.default_rng(3).uniform(-1, 0.5, c.ntotFine))
+    phi = _rand(c, 5, seed=4) / np.sqrt(c.ntot)
+    c.exx_setup(0.25, 0.0, 1, 6.0)
+    c.exx_set_phi(phi, np.ones(5))
+    c.exx_set_mode("full")
+    x = _rand(c, 3)
+    out = torch.empty_like(x)
+    g = c.capture_hpsi(x, out)
+    g.replay()
+    torch.cuda.synchronize()
+    ref = out.clone()
+    c.exx_apply(_rand(c, 64, seed=9))
+    from pwdft_develop_b200._lib import check, lib
+    check(lib.pw_exx_set_scratch(c.handle, 1 << 24))
+    y = torch.full((1 << 22,), 3.0, dtype=c.torch_dtype, device="cuda")
+    c.exx_apply(_rand(c, 70, seed=10))
+    out.zero_()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, ref) and bool((y == 3.0).all())
