@@ -299,6 +299,8 @@ struct Launch {
 inline bool nl_beside_chain(const pw_ctx* c) {
   return c->nl_mode == PW_NL_DENSE && c->have_nl && c->nproj > 0 && c->nl_overlap && !c->prof_on;
 }
+// room for a solver's blocks of npair band pairs (ctx.cu)
+void reserve_pairs(pw_ctx* c, int npair);
 // a coarse-spectrum table from the host: [kz][ky][kx] into dst and [kz][kx][ky] into dst_t
 int upload_spectrum(pw_ctx* c, DevBuf& dst, DevBuf& dst_t, const double* src);
 

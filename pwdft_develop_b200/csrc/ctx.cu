@@ -194,6 +194,10 @@ int ensure_scratch(pw_ctx* c, int npair) {
   return rc;
 }
 
+// a solver's request: at least npair pairs where there is room; it neither
+// narrows the batch nor counts as set by the caller
+void reserve_pairs(pw_ctx* c, int npair) { ensure_scratch(c, npair); }
+
 // after the projector tables changed: the batch again, halved until it fits
 int refit_scratch(pw_ctx* c) {
   int rc = PW_ENOMEM;

@@ -1359,7 +1359,7 @@ int pw_scf_run(pw_ctx* ctx, const pw_scf_params* p, pw_scf_result* r, double* ei
   if (p->mixed) {
     if (!ctx->twin && (rc = pw_ctx_build_twin(ctx))) return rc;
     S.c32 = ctx->twin;
-    if ((rc = pw_set_band_batch(S.c32, nb))) return rc;
+    reserve_pairs(S.c32, (nb + 1) / 2);
   }
   // CheFSI runs H*psi with the wavefunction cut-off filter at Ecut unless the
   // caller turns it off (KohnSham::Setup, hamiltonian.cpp:316-321); the
@@ -1391,7 +1391,7 @@ int pw_scf_run(pw_ctx* ctx, const pw_scf_params* p, pw_scf_result* r, double* ei
   for (double& x : g_sub) x = 0;
   double tph[6] = {0, 0, 0, 0, 0, 0};   // eigensolver, density, potentials, set-up, mixing, refine switch
   auto t_setup0 = std::chrono::steady_clock::now();
-  if ((rc = pw_set_band_batch(ctx, nb))) return rc;
+  reserve_pairs(ctx, (nb + 1) / 2);
   // device arrays
   for (DevBuf* b : {&S.rho, &S.rho_out, &S.rps, &S.vtot, &S.vtot_new, &S.vxc, &S.eps, &S.vh, &S.kern})
     if ((rc = b->alloc(nf * 8))) return rc;
@@ -2041,8 +2041,9 @@ int pw_ctx_build_twin(pw_ctx* ctx) {
   int rc = ctx->gs ? pw_ctx_create_gspace(ctx->L, ctx->nf, ctx->gs_ecut, PW_F32, ctx->device, &c32)
                    : pw_ctx_create(ctx->L, ctx->n, ctx->nf, PW_F32, ctx->device, &c32);
   if (rc) return rc;
-  if ((rc = pw_set_band_batch(c32, std::max(2, 2 * ctx->pair_cap))) ||
-      (rc = pw_set_atoms(c32, (int)ctx->atom_z.size(), ctx->atom_z.data(), ctx->atom_pos.data()))) {
+  if (ctx->batch_set) rc = pw_set_band_batch(c32, std::max(2, 2 * ctx->pair_cap));
+  else reserve_pairs(c32, ctx->pair_cap);
+  if (rc || (rc = pw_set_atoms(c32, (int)ctx->atom_z.size(), ctx->atom_z.data(), ctx->atom_pos.data()))) {
     pw_ctx_destroy(c32);
     return rc;
   }
@@ -2075,7 +2076,7 @@ int pw_eigsolve(pw_ctx* ctx, int solver, void* X, int nb, int maxit, double tol,
   Dense dn;
   int rc = dn.init((cublasHandle_t)ctx->blas);
   if (rc) return rc;
-  if ((rc = pw_set_band_batch(ctx, nb))) return rc;
+  reserve_pairs(ctx, (nb + 1) / 2);
   Solver sv;
   sv.c = ctx;
   sv.nt = ctx->ntot;

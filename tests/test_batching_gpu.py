@@ -178,3 +178,36 @@ def test_a_captured_exchange_outlives_larger_ones(mode, prec):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(out, ref) and bool((y == 3.0).all())
+
+
+def _count(c, f):
+    for _ in range(3):       # past any growth
+        f()
+    n = c.launches()
+    f()
+    return c.launches() - n
+
+
+@pytest.mark.parametrize("solver", ["eigsolve", "scf", "twin"])
+def test_a_solver_leaves_the_batch_to_the_calls(solver):
+    """After a narrow solve on the same context the wide calls and the k-point
+    batches take as many launches as on a fresh one."""
+    import torch
+    prec = "f32" if solver == "eigsolve" else "f64"
+    c, d = _ctx(prec), _ctx(prec)
+    if solver == "eigsolve":
+        c.eigsolve(_rand(c, 4) / np.sqrt(c.ntot), solver="lobpcg", maxit=2)
+    elif solver == "scf":
+        c.scf(nocc=16, nextra=4, ecut=5.0, solver="chebfsi", mixed=True, max_iter=2)
+    else:
+        c.build_twin()
+    x = _rand(c, 200)
+    ks = np.random.default_rng(1).uniform(-0.3, 0.3, (4, 3))
+    g = torch.Generator(device="cuda").manual_seed(2)
+    y = torch.view_as_complex(torch.randn((4, 24, c.ntot, 2), generator=g, device="cuda", dtype=x.dtype))
+    for e in (c, d):
+        e.set_vtot(np.linspace(-1, 0.5, c.ntotFine))
+        e.set_wfn_filter(None)
+        e.set_kpoints(ks)
+    for f in (lambda e: e.hpsi(x), lambda e: e.teter(x), lambda e: e.hpsi_kbatch(y)):
+        assert _count(c, lambda: f(c)) == _count(d, lambda: f(d))
