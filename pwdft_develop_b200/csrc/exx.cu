@@ -281,15 +281,7 @@ int pw_ace_apply(pw_ctx* ctx, const void* psi, int ld, void* out, int ldo, int n
   PWB_CHECK(ctx->ace_n > 0, PW_ENOTREADY, "ACE operator not built (pw_ace_build)");
   PWB_CUDA(cudaSetDevice(ctx->device));
   if (nband == 0) return PW_OK;
-  const int cap = std::max(1, 2 * ctx->pair_cap);
-  for (int b0 = 0; b0 < nband; b0 += cap) {
-    const int nb = std::min(cap, nband - b0);
-    const size_t e = ctx->esz;
-    int rc = run_ace(ctx, (const char*)psi + (size_t)b0 * ld * e, ld, nb, (char*)out + (size_t)b0 * ldo * e, ldo,
-                     (cudaStream_t)stream);
-    if (rc) return rc;
-  }
-  return PW_OK;
+  return run_ace(ctx, psi, ld, nband, out, ldo, (cudaStream_t)stream);
 }
 
 int pw_exx_energy(pw_ctx* ctx, const void* psi, int ld, int nband, const double* occ, int num_spin, int use_ace,

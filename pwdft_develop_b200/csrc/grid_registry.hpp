@@ -17,8 +17,8 @@ using DensFn = int (*)(pw_ctx*, const void*, int, int, int, int, const double*, 
 using TeterScratchFn = int (*)(pw_ctx*, const void*, int, void*, int, int, int, int, int, cudaStream_t, void*);
 using ExxFn = int (*)(pw_ctx*, const void*, int, int, void*, int, int, cudaStream_t);
 using HpsiKFn = int (*)(pw_ctx*, const void*, int, void*, int, int, int, int, cudaStream_t);
-using HpsiKBFn = int (*)(pw_ctx*, const void*, int, void*, int, int, int, int, cudaStream_t, int, const void*,
-                         const void*);
+using HpsiKBFn = int (*)(pw_ctx*, const void*, int, void*, int, int, int, int, cudaStream_t, int, const void*);
+using NlKFn = int (*)(pw_ctx*, const void*, int, void*, int, int, int, bool, cudaStream_t);
 using BuildQKFn = int (*)(pw_ctx*, const int*, const double*, const double*, const long*, const long*, const int*, int,
                           const double*, void*, cudaStream_t);
 
@@ -35,6 +35,7 @@ struct GridEntry {
   HpsiKFn hpsik[2];
   BuildQKFn bqk[2];
   HpsiKBFn hpsikb[2];
+  NlKFn nlk[2];
   HpsiFn hpsigs[2];     // sphere-cut (G-space) contexts whose G-space grid is twice this grid
   DensFn densgs[2];
 };

@@ -80,11 +80,17 @@ int run_hpsi_k(pw_ctx* c, const void* psi, int ld, void* out, int ldo, int band0
 }
 
 int run_hpsi_kbatch(pw_ctx* c, const void* psi, int ld, void* out, int ldo, int f0, int nf, int acc, cudaStream_t st,
-                    int fpk, const void* ekin_all, const void* qk_all) {
+                    int fpk, const void* ekin_all) {
   const GridEntry* g = find_grid(c->n);
   if (!g) { set_error("grid not built into this library"); return PW_EUNSUPPORTED; }
   if (gs_refuse(c, "the k-point batch")) return PW_EUNSUPPORTED;
-  return g->hpsikb[c->prec == PW_F32 ? 1 : 0](c, psi, ld, out, ldo, f0, nf, acc, st, fpk, ekin_all, qk_all);
+  return g->hpsikb[c->prec == PW_F32 ? 1 : 0](c, psi, ld, out, ldo, f0, nf, acc, st, fpk, ekin_all);
+}
+
+int run_nl_k(pw_ctx* c, const void* psi, int ld, void* out, int ldo, int nf, int fpk, bool all, cudaStream_t st) {
+  const GridEntry* g = find_grid(c->n);
+  if (!g) { set_error("grid not built into this library"); return PW_EUNSUPPORTED; }
+  return g->nlk[c->prec == PW_F32 ? 1 : 0](c, psi, ld, out, ldo, nf, fpk, all, st);
 }
 
 int run_build_q_k(pw_ctx* c, const int* d_idx, const double* d_beta, const double* d_disp, const long* d_pio,

@@ -71,7 +71,8 @@ static bool kq_tensor_cores(const pw_ctx* c) { return c->prec == PW_F32 && c->np
 
 int run_hpsi_k(pw_ctx* c, const void* psi, int ld, void* out, int ldo, int band0, int nb, int acc, cudaStream_t st);
 int run_hpsi_kbatch(pw_ctx* c, const void* psi, int ld, void* out, int ldo, int f0, int nf, int acc, cudaStream_t st,
-                    int fpk, const void* ekin_all, const void* qk_all);
+                    int fpk, const void* ekin_all);
+int run_nl_k(pw_ctx* c, const void* psi, int ld, void* out, int ldo, int nf, int fpk, bool all, cudaStream_t st);
 int run_build_q_k(pw_ctx* c, const int* d_idx, const double* d_beta, const double* d_disp, const long* d_pio,
                   const long* d_pbo, const int* d_pnp, int nproj, const double* kv, void* out, cudaStream_t st);
 int ensure_scratch(pw_ctx* c, int npair);
@@ -169,7 +170,7 @@ int pw_hpsi_k(pw_ctx* ctx, const void* psi, int ld, void* hpsi, int ldh, int nba
     int rc = run_hpsi_k(ctx, psi, ld, hpsi, ldh, b0, nb, accumulate, st);
     if (rc) return rc;
   }
-  return PW_OK;
+  return run_nl_k(ctx, psi, ld, hpsi, ldh, nband, nband, false, st);
 }
 
 int pw_set_kpoints(pw_ctx* ctx, int nk, const double* kpts) {
@@ -210,16 +211,14 @@ int pw_hpsi_kbatch(pw_ctx* ctx, const void* psi, int ld, void* hpsi, int ldh, in
   cudaStream_t st = (cudaStream_t)stream;
   const int nf = ctx->nkb * nband;
   if (nf == 0) return PW_OK;
-  int cap = batch_pairs(ctx, nf, st);
+  const int cap = batch_pairs(ctx, nf, st);
   if (cap < 1) return PW_ENOMEM;
-  if (cap > nband) cap -= cap % nband;   // whole k-points per batch
   for (int f0 = 0; f0 < nf; f0 += cap) {
     const int n = std::min(cap, nf - f0);
-    int rc = run_hpsi_kbatch(ctx, psi, ld, hpsi, ldh, f0, n, accumulate, st, nband, ctx->ekin_kb.p,
-                             ctx->nproj > 0 ? ctx->qkb.p : nullptr);
+    int rc = run_hpsi_kbatch(ctx, psi, ld, hpsi, ldh, f0, n, accumulate, st, nband, ctx->ekin_kb.p);
     if (rc) return rc;
   }
-  return PW_OK;
+  return run_nl_k(ctx, psi, ld, hpsi, ldh, nf, nband, true, st);
 }
 
 int pw_get_kpoint_tables(const pw_ctx* ctx, double* ekin_host, double* teter_host) {

@@ -43,6 +43,7 @@ namespace pwb {
 
 // bytes of one k-point's split-BF16 projector operands (kpoint.cu)
 size_t kq_bf_bytes(const pw_ctx* c);
+int wfn_filter_pass(pw_ctx* c, void* X, int ld, int nb, cudaStream_t st);
 
 // kx columns per z-pencil CTA: 24 for FP32 grids divisible by 24 (two
 // balanced tiles at n0 = 48), otherwise 16
@@ -1426,10 +1427,10 @@ struct Plan {
     // dense projector mode: Q D Q^T psi depends on psi only, so its GEMMs run
     // on a second stream while the FFT chain runs (their first output goes to
     // the rows of out, which the last coarse pass then accumulates into after
-    // the join), all bands of the call together (dense_call).  With pw_profile on
-    // the products run batch by batch after the chain, so each kernel is timed alone
-    const int nbnl = std::min(2 * npair, nband - band0);
-    const bool dense_nl = c->nl_mode == PW_NL_DENSE && c->have_nl && c->nproj > 0 && nbnl > 0;
+    // the join), all bands of the call together (dense_call).  With pw_profile on,
+    // and in FP64, they run after the chain of the last batch
+    const bool last = band0 + 2 * npair >= nband;
+    const bool dense_nl = c->nl_mode == PW_NL_DENSE && c->have_nl && c->nproj > 0;
     cudaStream_t sn = nullptr;
     if (dense_nl && nl_beside_chain(c)) {
       if (!c->nl_st) PWB_CUDA(cudaStreamCreateWithFlags(&c->nl_st, cudaStreamNonBlocking));
@@ -1453,10 +1454,7 @@ struct Plan {
       if (sn) PWB_CUDA(cudaStreamWaitEvent(st, c->nl_join, 0));
       reg_out<false>(c, out, ldo, nband, band0, npair, sn ? 1 : accumulate, st);
       PWB_CUDA(cudaGetLastError());
-      if (dense_nl && !sn)
-        if ((rc = dense_apply(c, nl_set(c, filt), psi + (long)band0 * ld, ld, out + (long)band0 * ldo, ldo, nbnl, st)))
-          return rc;
-      return exchange_batch(c, psi, ld, out, ldo, nband, band0, npair, st, filt);
+      return last ? call_tail(c, psi, ld, out, ldo, nband, dense_nl && !sn, st, filt) : PW_OK;
     }
     { Launch L_(c, st, KK_CXY_FWD);
     k_cxy_fwd<T, N0, N1><<<dim3(N2, npair), PLANE_THREADS, sm_cxy(), st>>>(psi, ld, nband, band0, AD, tw(c, 0), tw(c, 1)); }
@@ -1474,10 +1472,7 @@ struct Plan {
       k_cxy_inv<T, N0, N1><<<dim3(N2, npair), PLANE_THREADS, sm_cxy(), st>>>(AD, out, ldo, nband, band0,
                                                                           sn ? 1 : accumulate, tw(c, 0), tw(c, 1)); }
       PWB_CUDA(cudaGetLastError());
-      if (dense_nl && !sn)
-        if ((rc = dense_apply(c, nl_set(c, filt), psi + (long)band0 * ld, ld, out + (long)band0 * ldo, ldo, nbnl, st)))
-          return rc;
-      return exchange_batch(c, psi, ld, out, ldo, nband, band0, npair, st, filt);
+      return last ? call_tail(c, psi, ld, out, ldo, nband, dense_nl && !sn, st, filt) : PW_OK;
     }
     NLArgs nl{};
     const int cr = chunk_rows();
@@ -1514,30 +1509,40 @@ struct Plan {
     { Launch L_(c, st, KK_CXY_INV);
     k_cxy_inv<T, N0, N1><<<dim3(N2, npair), PLANE_THREADS, sm_cxy(), st>>>(AD, out, ldo, nband, band0, accumulate, tw(c, 0), tw(c, 1)); }
     PWB_CUDA(cudaGetLastError());
-    return exchange_batch(c, psi, ld, out, ldo, nband, band0, npair, st, filt);
+    return last ? call_tail(c, psi, ld, out, ldo, nband, false, st, filt) : PW_OK;
   }
 
-  // exact exchange of the batch's bands: the ACE operator (two GEMMs) or the
-  // full pair-FFT exchange, depending on the context's hybrid mode
-  static int exchange_batch(pw_ctx* c, const T* psi, int ld, T* out, int ldo, int nband, int band0, int npair,
-                            cudaStream_t st, bool filt = false) {
-    const int nb = std::min(2 * npair, nband - band0);
-    if (nb <= 0 || c->exx_mode == PW_EXX_OFF) return PW_OK;
-    if (c->exx_mode == PW_EXX_ACE) {
-      if (c->ace_n == 0) return PW_OK;
-      return dense_apply(c, ace_set(c, filt), psi + (long)band0 * ld, ld, out + (long)band0 * ldo, ldo, nb, st);
+  // what follows the batches of a call, for all its bands together: the dense
+  // projector products (unless they ran beside the chain) and the exchange.  They
+  // read the projector matrix (ACE vectors) once, and no result depends on how
+  // the bands were batched.
+  static int call_tail(pw_ctx* c, const T* psi, int ld, T* out, int ldo, int nband, bool dense, cudaStream_t st,
+                       bool filt = false) {
+    int rc;
+    if (dense && (rc = dense_call(c, nl_set(c, filt), psi, ld, out, ldo, nband, st))) return rc;
+    return exchange_call(c, psi, ld, out, ldo, nband, st, filt);
+  }
+
+  // exact exchange: the ACE operator (two GEMMs) or the full pair-FFT exchange,
+  // depending on the context's hybrid mode
+  static int exchange_call(pw_ctx* c, const T* psi, int ld, T* out, int ldo, int nband, cudaStream_t st, bool filt) {
+    if (c->exx_mode == PW_EXX_OFF) return PW_OK;
+    if (c->exx_mode == PW_EXX_ACE)
+      return c->ace_n == 0 ? PW_OK : dense_call(c, ace_set(c, filt), psi, ld, out, ldo, nband, st);
+    int rc;
+    if (c->gs) {
+      // 64 bands at a time: its full-grid workspaces go with the bands
+      for (int b0 = 0; b0 < nband; b0 += 64)
+        if ((rc = gs_exx_apply(c, psi + (long)b0 * ld, ld, std::min(64, nband - b0), out + (long)b0 * ldo, ldo, 1, st)))
+          return rc;
+      return PW_OK;
     }
-    if (c->gs) return gs_exx_apply(c, psi + (long)band0 * ld, ld, nb, out + (long)band0 * ldo, ldo, 1, st);
-    int rc = exx_apply(c, psi + (long)band0 * ld, ld, nb, out + (long)band0 * ldo, ldo, 1, st);
+    rc = exx_apply(c, psi, ld, nband, out, ldo, 1, st);
     if (rc || !filt) return rc;
     // the pair-FFT exchange has no fused filter: one explicit P pass over the
-    // batch's output bands (the local, kinetic and projector parts are already
-    // in the filtered space, and P is idempotent)
-    const void* saved = c->teter_tab;
-    c->teter_tab = c->wmask.p;
-    rc = teter_batch(c, out, ldo, out, ldo, nband, band0, npair, 0, st);
-    c->teter_tab = saved;
-    return rc;
+    // output bands (the local, kinetic and projector parts are already in the
+    // filtered space, and P is idempotent)
+    return wfn_filter_pass(c, out, ldo, nband, st);
   }
 
   // the projector matrix; with the filter the accumulating product reads P Q
@@ -1709,7 +1714,7 @@ struct Plan {
   // version, src/SCF/spinor_complex.cpp:292-542): one band per complex field,
   // idxFineGrid placement, kinetic 1/2 |k+G|^2, projectors with the Bloch phase
   static int hpsi_batch_k(pw_ctx* c, const V* psi, int ld, V* out, int ldo, int band0, int nb, int accumulate,
-                          cudaStream_t st, int fpk = 1 << 30, const T* ekin_all = nullptr, const V* qk_all = nullptr) {
+                          cudaStream_t st, int fpk = 1 << 30, const T* ekin_all = nullptr) {
     int rc = set_attrs();
     if (rc) return rc;
     static PerDeviceOnce attr;
@@ -1747,25 +1752,51 @@ struct Plan {
                                                                               band0, accumulate, tw(c, 0), tw(c, 1)); }
     }
     PWB_CUDA(cudaGetLastError());
-    if (c->nproj == 0 || !(qk_all ? qk_all : c->qk.p)) return PW_OK;
-    // V_nl psi = Q diag(d) Q^H psi with the complex coarse projector matrix Q of
-    // each k-point, one GEMM pair per k segment of the batch
-    const size_t kq_per = kq_bf_bytes(c);
+    return PW_OK;
+  }
+
+  // out += V_nl psi = Q diag(d) Q^H psi with the complex coarse projector matrix Q
+  // of each k-point, for all nf fields of a call (fpk bands per k-point; all: of
+  // the k-point batch, else of the one k-point), whatever its band batch is: FP32
+  // whole k-points together in even groups whose split bands take at most 512 MiB,
+  // halved while their operands find no room; FP64 one GEMM pair per k-point
+  static int nl_k_call(pw_ctx* c, const V* psi, int ld, V* out, int ldo, int nf, int fpk, bool all, cudaStream_t st) {
+    int rc;
+    if (c->nproj == 0 || !(all ? c->qkb.p : c->qk.p)) return PW_OK;
+    const int nk = nf / fpk;
     if constexpr (std::is_same<T, float>::value) {
-      // whole k-points of one batch together
-      const void* q0 = qk_all && c->qkb_bf.p ? (const char*)c->qkb_bf.p + (size_t)(band0 / fpk) * kq_per : nullptr;
-      if (q0 && band0 % fpk == 0 && nb % fpk == 0)
-        return nl_k_tc(c, q0, reinterpret_cast<const float*>(psi + (long)band0 * ld), ld,
-                       reinterpret_cast<float*>(out + (long)band0 * ldo), ldo, fpk, nb / fpk, st);
-    }
-    for (int f = band0; f < band0 + nb;) {
-      const int kk = f / fpk;
-      const int f1 = (int)std::min<long>(band0 + nb, (long)(kk + 1) * fpk);
-      const V* Qk = qk_all ? qk_all + (long)kk * c->nproj * c->ntot : reinterpret_cast<const V*>(c->qk.p);
-      const void* qbf = qk_all ? (c->qkb_bf.p ? (const char*)c->qkb_bf.p + (size_t)kk * kq_per : nullptr)
-                               : c->qk_bf.p;
-      if ((rc = nl_k(c, Qk, qbf, psi + (long)f * ld, ld, out + (long)f * ldo, ldo, f1 - f, st))) return rc;
-      f = f1;
+      const char* qbf = (const char*)(all ? c->qkb_bf.p : c->qk_bf.p);
+      if (!qbf) { set_error("k-point projector bf16 copies missing"); return PW_ENOTREADY; }
+      const size_t kq_per = kq_bf_bytes(c);
+      const int fmax = (int)std::max<long>(1, (512L << 20) / (8 * (long)c->ntot));
+      const int kmax = std::max(1, std::min(fmax / fpk, 65535));      // the reduction's grid
+      const int ngroup = (nk + kmax - 1) / kmax;
+      int kg = (nk + ngroup - 1) / ngroup, bg = fpk;
+      if (bg > fmax) bg = (fpk + (fpk + fmax - 1) / fmax - 1) / ((fpk + fmax - 1) / fmax);
+      for (int k0 = 0, b0 = 0; k0 < nk;) {
+        const int nkg = std::min(kg, nk - k0), nb = std::min(bg, fpk - b0);
+        const long f = (long)k0 * fpk + b0;
+        rc = nl_k_tc(c, qbf + (size_t)k0 * kq_per, reinterpret_cast<const float*>(psi + f * ld), ld,
+                     reinterpret_cast<float*>(out + f * ldo), ldo, nb, nkg, st);
+        if (rc == PW_ENOMEM && nkg * nb > 1) {
+          if (kg > 1) kg = (nkg + 1) / 2;
+          else bg = (nb + 1) / 2;
+          continue;
+        }
+        if (rc) return rc;
+        if (b0 + nb < fpk) {
+          b0 += nb;                 // kg is 1
+        } else {
+          b0 = 0;
+          k0 += nkg;
+        }
+      }
+    } else {
+      for (int kk = 0; kk < nk; ++kk) {
+        const V* Qk = reinterpret_cast<const V*>(all ? c->qkb.p : c->qk.p) + (long)kk * c->nproj * c->ntot;
+        const long f = (long)kk * fpk;
+        if ((rc = nl_k(c, Qk, psi + f * ld, ld, out + f * ldo, ldo, fpk, st))) return rc;
+      }
     }
     return PW_OK;
   }
@@ -1812,13 +1843,8 @@ struct Plan {
     return PW_OK;
   }
 
-  static int nl_k(pw_ctx* c, const V* Q, const void* qbf, const V* x, int ld, V* y, int ldo, int nb,
-                  cudaStream_t st) {
+  static int nl_k(pw_ctx* c, const V* Q, const V* x, int ld, V* y, int ldo, int nb, cudaStream_t st) {
     int rc;
-    if constexpr (std::is_same<T, float>::value) {
-      if (!qbf) { set_error("k-point projector bf16 copies missing"); return PW_ENOTREADY; }
-      return nl_k_tc(c, qbf, reinterpret_cast<const float*>(x), ld, reinterpret_cast<float*>(y), ldo, nb, 1, st);
-    } else {
     cublasHandle_t h = (cublasHandle_t)c->blas;
     if (cublasSetStream(h, st) != CUBLAS_STATUS_SUCCESS) { set_error("cublasSetStream failed"); return PW_ECUDA; }
     const int np = c->nproj, nt = (int)c->ntot;
@@ -1840,7 +1866,6 @@ struct Plan {
     if (r != CUBLAS_STATUS_SUCCESS) { set_error("projector GEMM (Q W) failed"); return PW_ECUDA; }
     PWB_CUDA(cudaGetLastError());
     return PW_OK;
-    }
   }
 
   // complex coarse projectors at Bloch vector k: q_l = T(conj(e^{i k.d}) beta_l),
@@ -1981,11 +2006,8 @@ struct Plan {
         BC, psi, ld, out, ldo, nband, band0, accumulate, reinterpret_cast<const int*>(c->gs_rows_fwd.p),
         reinterpret_cast<const int2*>(c->gs_ent_fwd.p), reinterpret_cast<const T*>(c->gs_ekin.p), tw(c, 5)); }
     PWB_CUDA(cudaGetLastError());
-    const int nb = std::min(2 * npair, nband - band0);
-    if (c->have_nl && c->nproj > 0 && nb > 0 &&
-        (rc = dense_apply(c, nl_set(c), psi + (long)band0 * ld, ld, out + (long)band0 * ldo, ldo, nb, st)))
-      return rc;
-    return exchange_batch(c, psi, ld, out, ldo, nband, band0, npair, st);
+    if (band0 + 2 * npair < nband) return PW_OK;
+    return call_tail(c, psi, ld, out, ldo, nband, c->have_nl && c->nproj > 0, st);
   }
 
   // rho += sum of w_b |psi_b(r)|^2 from sphere coefficients (CalculateDensity
@@ -2049,8 +2071,8 @@ static int exx_thunk(pw_ctx* c, const void* psi, int ld, int nb, void* out, int 
 template <typename T, int N0, int N1, int N2>
 static int ace_thunk(pw_ctx* c, const void* psi, int ld, int nb, void* out, int ldo, int acc, cudaStream_t st) {
   (void)acc;
-  return Plan<T, N0, N1, N2>::dense_apply(c, Plan<T, N0, N1, N2>::ace_set(c), (const T*)psi, ld, (T*)out, ldo, nb,
-                                          st);
+  return Plan<T, N0, N1, N2>::dense_call(c, Plan<T, N0, N1, N2>::ace_set(c), (const T*)psi, ld, (T*)out, ldo, nb,
+                                         st);
 }
 
 template <typename T, int N0, int N1, int N2>
@@ -2061,10 +2083,16 @@ static int hpsik_thunk(pw_ctx* c, const void* psi, int ld, void* out, int ldo, i
 }
 template <typename T, int N0, int N1, int N2>
 static int hpsikb_thunk(pw_ctx* c, const void* psi, int ld, void* out, int ldo, int band0, int nb, int acc,
-                        cudaStream_t st, int fpk, const void* ekin_all, const void* qk_all) {
+                        cudaStream_t st, int fpk, const void* ekin_all) {
   using V = VT<T>;
   return Plan<T, N0, N1, N2>::hpsi_batch_k(c, (const V*)psi, ld, (V*)out, ldo, band0, nb, acc, st, fpk,
-                                           (const T*)ekin_all, (const V*)qk_all);
+                                           (const T*)ekin_all);
+}
+template <typename T, int N0, int N1, int N2>
+static int nlk_thunk(pw_ctx* c, const void* psi, int ld, void* out, int ldo, int nf, int fpk, bool all,
+                     cudaStream_t st) {
+  using V = VT<T>;
+  return Plan<T, N0, N1, N2>::nl_k_call(c, (const V*)psi, ld, (V*)out, ldo, nf, fpk, all, st);
 }
 template <typename T, int N0, int N1, int N2>
 static int hpsigs_thunk(pw_ctx* c, const void* psi, int ld, void* out, int ldo, int nband, int band0, int npair,
@@ -2094,6 +2122,7 @@ static int buildqk_thunk(pw_ctx* c, const int* a, const double* b, const double*
    {hpsik_thunk<double, a, b, c>, hpsik_thunk<float, a, b, c>},                                    \
    {buildqk_thunk<double, a, b, c>, buildqk_thunk<float, a, b, c>},                                \
    {hpsikb_thunk<double, a, b, c>, hpsikb_thunk<float, a, b, c>},                                  \
+   {nlk_thunk<double, a, b, c>, nlk_thunk<float, a, b, c>},                                        \
    {hpsigs_thunk<double, a, b, c>, hpsigs_thunk<float, a, b, c>},                                  \
    {densgs_thunk<double, a, b, c>, densgs_thunk<float, a, b, c>}}
 

@@ -36,9 +36,8 @@ def test_batch_follows_the_call(nb):
     ref = torch.cat([c.teter(x[i:i + 2]) for i in range(0, nb, 2)])
     assert torch.equal(c.teter(x), ref)
     assert torch.equal(d.teter(x), ref)
-    # the FP64 projector products are a library's: equal to rounding only
-    a, b = c.hpsi(x), d.hpsi(x)
-    assert (a - b).abs().max() <= 1e-13 * a.abs().max()
+    # the projector products take all bands of a call, however they are batched
+    assert torch.equal(c.hpsi(x), d.hpsi(x))
 
 
 def test_a_captured_call_outlives_larger_ones():
@@ -63,7 +62,8 @@ def test_a_captured_call_outlives_larger_ones():
 @pytest.mark.parametrize("batch", [None, 2, 10, 22, 30])
 def test_kpoint_batches(prec, batch):
     """nk = 5 of nb = 7: all together, whole k-points per batch (22, 30 fields)
-    and k-points cut by the batch (1, 5 fields)."""
+    and k-points cut by the batch (1, 5 fields); the projector products take
+    whole k-points in all of them, so the bits are those of one batch."""
     import torch
     c = _ctx(prec)
     if batch:
@@ -76,6 +76,9 @@ def test_kpoint_batches(prec, batch):
     x = torch.randn((5, 7, c.ntot, 2), generator=g, device="cuda", dtype=torch.float64)
     x = torch.view_as_complex(x).to(ct)
     got = c.hpsi_kbatch(x)
+    if batch:
+        c.set_band_batch(2 * 5 * 7)
+        assert torch.equal(got, c.hpsi_kbatch(x))
     for i, k in enumerate(ks):
         c.set_kpoint(k)
         ref = c.hpsi_k(x[i].contiguous())
@@ -211,3 +214,39 @@ def test_a_solver_leaves_the_batch_to_the_calls(solver):
         e.set_kpoints(ks)
     for f in (lambda e: e.hpsi(x), lambda e: e.teter(x), lambda e: e.hpsi_kbatch(y)):
         assert _count(c, lambda: f(c)) == _count(d, lambda: f(d))
+
+
+@pytest.mark.parametrize("mode", ["sphere", "serial", "full", "full filter", "ace"])
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+def test_no_result_depends_on_the_batch(mode, prec):
+    """Serial and sphere-cut projector products and the exchange after them: the
+    bits of one batch in batches of 3 pairs, accumulated or not."""
+    import torch
+    if mode == "sphere":
+        from oracle import pw
+        from pwdft_develop_b200 import Context
+        L, z, pos = pw.make_crystal("Si", (1, 1, 1), A, 0.02, 77)
+        c = Context.gspace(L, (32, 32, 32), 6.0, precision=prec)
+        c.set_atoms([z] * len(pos), pos)
+        c.set_vtot(np.random.default_rng(3).uniform(-1, 0.5, c.ntotFine))
+    else:
+        c = _ctx(prec)
+    if mode == "serial":
+        from pwdft_develop_b200._lib import check, lib
+        check(lib.pw_set_nl_overlap(c.handle, 0))
+    x = _rand(c, 25) / np.sqrt(c.ntot)
+    if mode != "serial":
+        phi = _rand(c, 30, seed=4) / np.sqrt(c.ntot)
+        c.exx_setup(0.25, 0.0, 1, 6.0)
+        c.exx_set_phi(phi, np.ones(30))
+        c.exx_set_mode("full")
+    if mode == "ace":
+        c.ace_build(phi)
+    if mode == "full filter":
+        c.set_wfn_filter(5.0)
+    c.set_band_batch(26)
+    base = torch.randn_like(x)
+    ref, refa = c.hpsi(x), c.hpsi(x, out=base.clone(), accumulate=True)
+    c.set_band_batch(6)
+    assert torch.equal(c.hpsi(x), ref)
+    assert torch.equal(c.hpsi(x, out=base.clone(), accumulate=True), refa)
