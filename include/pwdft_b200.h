@@ -560,9 +560,15 @@ PW_API int pw_scf_forces(pw_ctx* ctx, double* force, double* force_local, double
 PW_API int pw_teter_precond_noalloc(pw_ctx* ctx, const void* r, int ld, void* w, int ldw, int nband, int accumulate,
                                     void* stream);
 
-/* Maximum number of bands processed per internal batch (sets scratch size).
- * Until this is called the batch follows the calls (scratch grows to the widest
- * block, at most 640 MiB); afterwards it stays as set. */
+/* Maximum number of bands processed per internal batch (sets the size of the
+ * H*psi scratch).  Until this is called the batch follows the calls: a call wider
+ * than the scratch runs in batches, a second one grows it, to at most 640 MiB
+ * (blocks that a later call outgrows stay until the context ends, because a
+ * captured graph may read them: all blocks together hold less than three times
+ * that).  Afterwards the batch stays as set, except that pw_scf_run and
+ * pw_eigsolve make room for their own bands, and pw_autotune sets the width it
+ * finds.  The dense projector products take all bands of a call, in groups of
+ * at most 512 MiB of split operands, whatever the batch. */
 PW_API int pw_set_band_batch(pw_ctx* ctx, int nband_batch);
 
 /* ---- Restart files in the reference's binary layout ----

@@ -223,6 +223,9 @@ struct pw_ctx {
   // scratch for the band-pair pipeline
   int pair_cap = 0;
   bool batch_set = false;          // pw_set_band_batch was called (or a growth refused): the batch stays
+  // an H*psi (k-point, Teter) call wider than its scratch came by since the last
+  // growth: the next one grows it (batch_pairs)
+  bool wide_hpsi = false, wide_teter = false, grown = false;
   // blocks of the H*psi scratch outgrown by a later call: a graph captured before
   // may still read them, so they live as long as the context
   std::vector<void*> retired;

@@ -170,25 +170,30 @@ int prepare_wfn_filter(pw_ctx* c) {
   return PW_OK;
 }
 
+// elements of one band pair in the blocks of the H*psi scratch: slot fields,
+// coarse fields (twice: spectra and kinetic term; the sphere-cut path has none)
+// and the real-space projectors' sums per slot and per atom
+static size_t pair_slots(const pw_ctx* c) { return (size_t)c->nf[2] * (c->n[1] + 1) * (c->n[0] + 1); }
+static size_t pair_coarse(const pw_ctx* c) { return c->gs ? 0 : (size_t)c->ntot; }
+static size_t pair_wp(const pw_ctx* c) { return (size_t)std::max(1, c->nl.nslot) * std::max(1, c->nl.npmax); }
+static size_t pair_w(const pw_ctx* c) { return (size_t)std::max(1, c->nl.natom) * std::max(1, c->nl.npmax); }
+
 // room for npair pairs in every block of the H*psi scratch; a failure leaves the
 // blocks that were there (or grew already)
 static int alloc_scratch(pw_ctx* c, int npair) {
-  const size_t cs = 2 * c->esz;   // complex element
-  const size_t nb = (size_t)c->nf[2] * (c->n[1] + 1) * (c->n[0] + 1);
+  const size_t pairs = (size_t)npair * 2 * c->esz;   // complex elements
   int rc;
   // the largest first: a growth that does not fit then takes nothing
-  if ((rc = c->s_bc.alloc((size_t)npair * nb * cs))) return rc;
-  if ((rc = c->s_ad.alloc((size_t)npair * c->ntot * cs))) return rc;
-  if ((rc = c->s_k.alloc((size_t)npair * c->ntot * cs))) return rc;
-  const size_t nslot = std::max(1, c->nl.nslot), nat = std::max(1, c->nl.natom), np = std::max(1, c->nl.npmax);
-  if ((rc = c->s_wp.alloc((size_t)npair * nslot * np * cs))) return rc;
-  if ((rc = c->s_w.alloc((size_t)npair * nat * np * cs))) return rc;
-  return c->s_wq.grow((size_t)std::max(1, c->nproj) * 2 * npair * c->esz);
+  if ((rc = c->s_bc.alloc(pairs * pair_slots(c)))) return rc;
+  if ((rc = c->s_ad.alloc(pairs * pair_coarse(c)))) return rc;
+  if ((rc = c->s_k.alloc(pairs * pair_coarse(c)))) return rc;
+  if ((rc = c->s_wp.alloc(pairs * pair_wp(c)))) return rc;
+  return c->s_w.alloc(pairs * pair_w(c));
 }
 
 // at least npair pairs; a failure leaves the batch as it was
 int ensure_scratch(pw_ctx* c, int npair) {
-  if (npair <= c->pair_cap && c->s_ad.p) return PW_OK;
+  if (npair <= c->pair_cap) return PW_OK;
   const int rc = alloc_scratch(c, npair);
   if (!rc) c->pair_cap = npair;
   return rc;
@@ -208,26 +213,46 @@ int refit_scratch(pw_ctx* c) {
   return rc;
 }
 
+// the pairs whose H*psi scratch 640 MiB hold (wider batches gained nothing)
+static int batch_limit(const pw_ctx* c) {
+  const size_t per = (pair_slots(c) + 2 * pair_coarse(c) + (c->nl.nslot > 0 ? pair_wp(c) + pair_w(c) : 0)) * 2 * c->esz;
+  return (int)std::min<size_t>(1 << 30, std::max<size_t>(1, ((size_t)640 << 20) / per));
+}
+
 // The band batch follows the calls: one launch per pass over all `npair` fields
-// where the batch fields fit in 640 MiB (a new block costs
-// its first call about 7 ms per GB); Si64, 80 pairs: the five passes take
-// 400 us in one batch and 436 us in batches of 32, and the projector matrix
-// is read once, not three times).  It stays as it is once the caller has set it,
-// once a growth was refused, and in a call that is being captured.  The passes
-// then split the bands evenly.
-int batch_pairs(pw_ctx* c, int npair, cudaStream_t st) {
-  if (npair > c->pair_cap && !c->batch_set) {
-    const size_t per = (2 * (size_t)c->ntot + (size_t)c->nf[2] * (c->n[1] + 1) * (c->n[0] + 1)) * 2 * c->esz;
-    const int want = (int)std::min<size_t>(npair, ((size_t)640 << 20) / per);
+// where they fit in batch_limit pairs (Si64, 80 pairs: the five passes take
+// 400 us in one batch and 436 us in batches of 32).  New blocks cost about 7 ms per
+// GB, which one call does not earn back, so the first call that is wider than
+// the scratch runs in the batches that are there and the second one grows it:
+// to its own width, later to at least twice what there is (all blocks, outgrown
+// ones included, then stay below three times the limit).  Teter grows its own
+// block alone, and needs none in the sphere-cut mode.  The batch stays as it is
+// once the caller has set it, once a growth was refused, and in a call that is
+// being captured.  The passes split the bands evenly.
+int batch_pairs(pw_ctx* c, int npair, cudaStream_t st, bool teter) {
+  if (teter && c->gs) return npair;
+  const size_t coarse = (size_t)c->ntot * 2 * c->esz;
+  auto cap = [&] { return teter && !c->batch_set ? std::max(c->pair_cap, (int)(c->s_ad.bytes / coarse)) : c->pair_cap; };
+  const int want = std::min(npair, batch_limit(c));
+  if (want > cap() && !c->batch_set) {
+    bool& seen = teter ? c->wide_teter : c->wide_hpsi;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-    if (want > c->pair_cap && cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
+    if (seen && cudaStreamIsCapturing(st, &cs) != cudaSuccess) {
       cudaGetLastError();
       cs = cudaStreamCaptureStatusActive;
     }
-    if (want > c->pair_cap && cs == cudaStreamCaptureStatusNone && ensure_scratch(c, want)) c->batch_set = true;
+    if (seen && cs == cudaStreamCaptureStatusNone) {
+      const int to = c->grown ? std::max(want, std::min(2 * cap(), batch_limit(c))) : want;
+      if (teter ? c->s_ad.alloc(to * coarse) : ensure_scratch(c, to)) c->batch_set = true;
+      c->grown = true;
+      seen = false;
+    } else {
+      seen = true;
+    }
   }
-  if (c->pair_cap < 1) return 0;
-  const int nb = (npair + c->pair_cap - 1) / c->pair_cap;
+  const int have = cap();
+  if (have < 1) return 0;
+  const int nb = (npair + have - 1) / have;
   return (npair + nb - 1) / std::max(1, nb);
 }
 
@@ -593,8 +618,8 @@ int pw_hpsi(pw_ctx* ctx, const void* psi, int ld, void* hpsi, int ldh, int nband
     if (rc) return rc;
   }
   if (nband == 0) return PW_OK;
-  const int cap = batch_pairs(ctx, (nband + 1) / 2, st);
-  if (cap < 1) return PW_ENOMEM;
+  const int cap = batch_pairs(ctx, (nband + 1) / 2, st, false);
+  PWB_CHECK(cap > 0, PW_ENOMEM, "no device scratch");
   for (int b0 = 0; b0 < nband; b0 += 2 * cap) {
     const int npair = std::min(cap, (nband - b0 + 1) / 2);
     int rc = run_hpsi(ctx, psi, ld, hpsi, ldh, nband, b0, npair, accumulate, st);
@@ -675,8 +700,8 @@ int pw_teter_precond(pw_ctx* ctx, const void* r, int ld, void* w, int ldw, int n
   PWB_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t st = (cudaStream_t)stream;
   if (nband == 0) return PW_OK;
-  const int cap = batch_pairs(ctx, (nband + 1) / 2, st);
-  if (cap < 1) return PW_ENOMEM;
+  const int cap = batch_pairs(ctx, (nband + 1) / 2, st, true);
+  PWB_CHECK(cap > 0, PW_ENOMEM, "no device scratch");
   for (int b0 = 0; b0 < nband; b0 += 2 * cap) {
     const int npair = std::min(cap, (nband - b0 + 1) / 2);
     int rc = run_teter(ctx, r, ld, w, ldw, nband, b0, npair, accumulate, st);

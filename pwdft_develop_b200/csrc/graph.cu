@@ -28,6 +28,8 @@ int pw_graph_capture_hpsi(pw_ctx* ctx, const void* psi, int ld, void* hpsi, int 
   PWB_CHECK(!ctx->prof_on, PW_EINVAL, "per-kernel profiling is on (pw_profile); graphs need it off");
   PWB_CUDA(cudaSetDevice(ctx->device));
   // warm-up outside the capture: scratch, kernel attributes, library handles
+  // (with the batch that repeated calls of this width would grow to)
+  ctx->wide_hpsi = true;
   int rc = pw_hpsi(ctx, psi, ld, hpsi, ldh, nband, accumulate, nullptr);
   if (rc) return rc;
   PWB_CUDA(cudaDeviceSynchronize());
@@ -116,6 +118,7 @@ int pw_graph_capture_batch(int ncell, pw_ctx* const* ctxs, const void* const* ps
   PWB_CHECK(graph, PW_EINVAL, "null argument");
   PWB_CUDA(cudaSetDevice(ctxs[0]->device));
   // warm-up outside the capture (scratch, attributes, library handles)
+  for (int c = 0; c < ncell; ++c) ctxs[c]->wide_hpsi = true;
   if ((rc = batch_enqueue(ncell, ctxs, psi, ld, out, ldo, nband, nullptr))) return rc;
   PWB_CUDA(cudaDeviceSynchronize());
   std::vector<char> chk(ncell);

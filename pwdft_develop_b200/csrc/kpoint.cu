@@ -76,7 +76,7 @@ int run_nl_k(pw_ctx* c, const void* psi, int ld, void* out, int ldo, int nf, int
 int run_build_q_k(pw_ctx* c, const int* d_idx, const double* d_beta, const double* d_disp, const long* d_pio,
                   const long* d_pbo, const int* d_pnp, int nproj, const double* kv, void* out, cudaStream_t st);
 int ensure_scratch(pw_ctx* c, int npair);
-int batch_pairs(pw_ctx* c, int npair, cudaStream_t st);
+int batch_pairs(pw_ctx* c, int npair, cudaStream_t st, bool teter);
 int upload_real(pw_ctx* c, DevBuf& dst, const double* src, size_t n);
 
 template <typename X> static int upload(DevBuf& b, const std::vector<X>& h) {
@@ -163,8 +163,8 @@ int pw_hpsi_k(pw_ctx* ctx, const void* psi, int ld, void* hpsi, int ldh, int nba
   PWB_CUDA(cudaSetDevice(ctx->device));
   cudaStream_t st = (cudaStream_t)stream;
   if (nband == 0) return PW_OK;
-  const int cap = batch_pairs(ctx, nband, st);
-  if (cap < 1) return PW_ENOMEM;
+  const int cap = batch_pairs(ctx, nband, st, false);
+  PWB_CHECK(cap > 0, PW_ENOMEM, "no device scratch");
   for (int b0 = 0; b0 < nband; b0 += cap) {
     const int nb = std::min(cap, nband - b0);
     int rc = run_hpsi_k(ctx, psi, ld, hpsi, ldh, b0, nb, accumulate, st);
@@ -211,8 +211,8 @@ int pw_hpsi_kbatch(pw_ctx* ctx, const void* psi, int ld, void* hpsi, int ldh, in
   cudaStream_t st = (cudaStream_t)stream;
   const int nf = ctx->nkb * nband;
   if (nf == 0) return PW_OK;
-  const int cap = batch_pairs(ctx, nf, st);
-  if (cap < 1) return PW_ENOMEM;
+  const int cap = batch_pairs(ctx, nf, st, false);
+  PWB_CHECK(cap > 0, PW_ENOMEM, "no device scratch");
   for (int f0 = 0; f0 < nf; f0 += cap) {
     const int n = std::min(cap, nf - f0);
     int rc = run_hpsi_kbatch(ctx, psi, ld, hpsi, ldh, f0, n, accumulate, st, nband, ctx->ekin_kb.p);

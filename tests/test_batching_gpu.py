@@ -250,3 +250,79 @@ def test_no_result_depends_on_the_batch(mode, prec):
     c.set_band_batch(6)
     assert torch.equal(c.hpsi(x), ref)
     assert torch.equal(c.hpsi(x, out=base.clone(), accumulate=True), refa)
+
+
+def _grown(f):
+    """Device memory that a call takes and keeps."""
+    import torch
+    torch.cuda.synchronize()
+    a = torch.cuda.mem_get_info()[0]
+    f()
+    torch.cuda.synchronize()
+    return a - torch.cuda.mem_get_info()[0]
+
+
+def test_one_wide_call_takes_no_new_scratch():
+    """The first call wider than the scratch runs in the batches that are there,
+    with the bits of the later ones; the second takes what it needs, Teter its
+    one block of coarse fields; a narrower call takes nothing."""
+    import torch
+    c, w = _ctx("f64", n=(24, 24, 24)), _ctx("f64", n=(24, 24, 24))
+    c.set_band_batch(64)         # w's: the kernels and library handles of both calls are there
+    x = _rand(c, 200)
+    out, wout = torch.empty_like(x), torch.empty_like(x)
+    c.hpsi(x, out=out), c.teter(x, out=out)
+    pair = 16 * (2 * 24 ** 3 + 48 * 25 * 25)
+    assert _grown(lambda: w.teter(x, out=wout)) < 4 << 20
+    first = wout.clone()
+    coarse = 100 * 16 * 24 ** 3
+    assert coarse <= _grown(lambda: w.teter(x, out=wout)) < coarse + (4 << 20)
+    assert torch.equal(wout, first)
+    assert _grown(lambda: w.hpsi(x, out=wout)) < 4 << 20
+    first = wout.clone()
+    rest = 100 * pair - coarse
+    assert rest <= _grown(lambda: w.hpsi(x, out=wout)) < rest + (6 << 20)
+    assert torch.equal(wout, first)
+    assert _grown(lambda: (w.hpsi(x, out=wout), w.teter(x[:150], out=wout[:150]))) == 0
+
+
+def test_the_scratch_stays_within_its_limit():
+    """Ever wider calls: the blocks in use hold at most 640 MiB, all of them less
+    than three times that, and the batch no longer grows there."""
+    import torch
+    c = _ctx("f64", n=(24, 24, 24))
+    c.set_atoms([14], [(0.0, 0.0, 0.0)])
+    x = _rand(c, 3000)
+    out = torch.empty_like(x)
+    pair = 16 * (2 * 24 ** 3 + 48 * 25 * 25)
+    lim = (640 << 20) // pair
+    c.hpsi(x[:66], out=out[:66])
+
+    def grow():
+        for nb in range(80, 3000, 40):
+            c.hpsi(x[:nb], out=out[:nb])
+    assert _grown(grow) < 3 * (640 << 20)
+    n = c.launches()
+    c.hpsi(x, out=out)
+    batches = -(-1500 // lim)
+    assert c.launches() - n == 5 * batches + 1
+
+
+def test_sphere_cut_scratch():
+    """Sphere-cut calls take slot fields alone, and Teter nothing."""
+    import torch
+    from oracle import pw
+    from pwdft_develop_b200 import Context
+    L, z, pos = pw.make_crystal("Si", (1, 1, 1), A, 0.02, 77)
+    c = Context.gspace(L, (48, 48, 48), 10.0, precision="f64")
+    c.set_vtot(np.random.default_rng(3).uniform(-1, 0.5, c.ntotFine))
+    x = _rand(c, 200)
+    out = torch.empty_like(x)
+    c.hpsi(x[:8], out=out[:8])
+    c.teter(x[:8], out=out[:8])
+    assert _grown(lambda: (c.teter(x, out=out), c.teter(x, out=out))) == 0
+    assert _grown(lambda: c.hpsi(x, out=out)) == 0
+    first = out.clone()
+    slots = 100 * 16 * 48 * 25 * 25
+    assert slots <= _grown(lambda: c.hpsi(x, out=out)) < slots + (4 << 20)
+    assert torch.equal(out, first)
