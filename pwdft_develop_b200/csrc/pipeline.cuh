@@ -1868,6 +1868,14 @@ struct Plan {
     return PW_OK;
   }
 
+  // complex fine fields per pass of a projector build: no more than there are, than
+  // the scratch holds, than 32 and than 512 MiB (the fields are temporary, and
+  // memory costs its allocation about 7 ms per GB)
+  static int build_cap(const pw_ctx* c, int nfield) {
+    const size_t fmax = ((size_t)512 << 20) / (2 * (size_t)c->ntotf * sizeof(T));
+    return std::min(std::min(c->pair_cap, nfield), (int)std::min<size_t>(32, std::max<size_t>(1, fmax)));
+  }
+
   // complex coarse projectors at Bloch vector k: q_l = T(conj(e^{i k.d}) beta_l),
   // one projector per complex field, into Qout (complex, leading dimension ntot)
   static int build_q_k(pw_ctx* c, const int* d_idx, const double* d_beta, const double* d_disp, const long* d_pio,
@@ -1879,7 +1887,8 @@ struct Plan {
       PWB_CUDA(cudaFuncSetAttribute(k_cxy_inv<T, N0, N1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_cxy()));
       attr.mark();
     }
-    const int cap = c->pair_cap;                 // complex fields per pass
+    const int cap = build_cap(c, nproj);         // complex fields per pass
+    PWB_CHECK(cap > 0, PW_ENOMEM, "no device scratch");
     const long nf = c->ntotf;
     DevBuf fields;
     if ((rc = fields.alloc((size_t)2 * cap * nf * sizeof(T)))) return rc;
@@ -1909,7 +1918,8 @@ struct Plan {
                      const int* d_pnp, int nproj, cudaStream_t st, int deriv = 0, T* Qout = nullptr) {
     int rc = set_attrs();
     if (rc) return rc;
-    const int cap = c->pair_cap;                 // pairs per pass
+    const int cap = build_cap(c, (nproj + 1) / 2);   // pairs per pass
+    PWB_CHECK(cap > 0, PW_ENOMEM, "no device scratch");
     const long nf = c->ntotf;
     DevBuf fields;
     if ((rc = fields.alloc((size_t)2 * cap * nf * sizeof(T)))) return rc;

@@ -326,3 +326,28 @@ def test_sphere_cut_scratch():
     slots = 100 * 16 * 48 * 25 * 25
     assert slots <= _grown(lambda: c.hpsi(x, out=out)) < slots + (4 << 20)
     assert torch.equal(out, first)
+
+
+def test_projector_builds_take_fields_for_their_projectors():
+    """After a wide k-point batch the temporary fields of a build still go with
+    the projectors: there is room for them on a nearly full device."""
+    import torch
+    c, d = _ctx("f32", n=(24, 24, 24)), _ctx("f32", n=(24, 24, 24))
+    ks = np.random.default_rng(1).uniform(-0.3, 0.3, (4, 3))
+    c.set_kpoints(ks)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    y = torch.view_as_complex(torch.randn((4, 300, c.ntot, 2), generator=g, device="cuda"))
+    for _ in range(3):
+        c.hpsi_kbatch(y)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (200 << 20), dtype=torch.uint8, device="cuda")
+    c.set_kpoint(ks[1] / 2)
+    from oracle import pw
+    _, z, pos = pw.make_crystal("Si", (1, 1, 1), A, 0.02, 77)
+    c.set_atoms([z] * len(pos), pos)
+    del fill
+    torch.cuda.empty_cache()
+    d.set_kpoint(ks[1] / 2)
+    x = y[0, :5].contiguous()
+    assert torch.equal(c.hpsi_k(x), d.hpsi_k(x))
