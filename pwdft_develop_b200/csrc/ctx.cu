@@ -188,7 +188,9 @@ static int alloc_scratch(pw_ctx* c, int npair) {
   if ((rc = c->s_ad.alloc(pairs * pair_coarse(c)))) return rc;
   if ((rc = c->s_k.alloc(pairs * pair_coarse(c)))) return rc;
   if ((rc = c->s_wp.alloc(pairs * pair_wp(c)))) return rc;
-  return c->s_w.alloc(pairs * pair_w(c));
+  if ((rc = c->s_w.alloc(pairs * pair_w(c)))) return rc;
+  // the projections of as many bands (FP64; a wider call grows them)
+  return c->prec == PW_F64 ? c->s_wq.grow((size_t)c->nproj * 2 * npair * c->esz) : PW_OK;
 }
 
 // at least npair pairs; a failure leaves the batch as it was
