@@ -552,6 +552,7 @@ template <int BN> static int launch_bn(const SplitOperand& A, const SplitOperand
     for (int nt = 0; nt < tilesN; ++nt) ga.ntiles += sym_tiles_in_col(nt, BN, tilesM);
   }
   const long total = (long)(ga.sym ? ga.ntiles : tilesM * tilesN) * nsplit * ga.nbatch;
+  PWB_CHECK(total < (1L << 31), PW_EUNSUPPORTED, "too many tiles in one batched product");
   const int grid = (int)std::min<long>(total, num_sms());
   k_gemm_tn<BN><<<grid, GEMM_THREADS, SM::BYTES, st>>>(ah, al, bh, bl, ga);
   PWB_CUDA(cudaGetLastError());
@@ -629,6 +630,7 @@ int split_bf16_t(const float* x, long ld_in, int ncol, int nrow, void* hi, void*
 int gemm_tn_reduce(const SplitOperand& A, const SplitOperand& B, int K, int nterms, DevBuf& ws,
                    const ReduceOut& out, cudaStream_t st, int bn, int sym, int nbatch) {
   const int M = A.rows, N = B.rows;
+  PWB_CHECK(reduce_ok(out, nbatch), PW_EINVAL, "batched reduction without a place for each product");
   if (M == 0 || N == 0) return PW_OK;
   const int BN = bn > 0 ? bn : pick_bn(N);
   sym = sym && M == N;

@@ -30,11 +30,17 @@ struct ReduceOut {
   long bs_bf = 0;   // elements of bf_hi / bf_lo from one batch item to the next
 };
 
+// what a reduction of nbatch products cannot write: `out` has one product's
+// place, overlapping bf16 rows, and a grid dimension takes 65535 products
+inline bool reduce_ok(const ReduceOut& out, int nbatch) {
+  return nbatch == 1 || (nbatch > 0 && nbatch <= 65535 && !out.out && (!out.bf_hi || out.bs_bf > 0));
+}
+
 int split_bf16(const float* x, long ld_in, int ncol, int nrow, void* hi, void* lo, long ld_out, float scale,
                cudaStream_t st);
 int split_bf16_t(const float* x, long ld_in, int ncol, int nrow, void* hi, void* lo, long ld_out, cudaStream_t st);
 // nbatch products of one shape in one launch (k-points: 64 launches of a few us
-// each otherwise); a batched reduction writes the bf16 pair only
+// each otherwise); a batched reduction writes the bf16 pair only (reduce_ok)
 // C[m][n] = sum_k A[m][k] B[n][k] with split-K and a deterministic reduction
 // bn: tile width override (0 = heuristic; otherwise one of 32, 64, 96, 128, 160, 192, 256)
 // sym: A and B are the same operand (a symmetric product): only the tiles not

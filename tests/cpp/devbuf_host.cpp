@@ -5,6 +5,7 @@
 #include <map>
 
 #include "../../pwdft_develop_b200/csrc/devbuf.cpp"
+#include "../../pwdft_develop_b200/csrc/gemm.hpp"
 
 static std::map<void*, size_t> g_live;
 static size_t g_used = 0, g_limit = 0;
@@ -98,6 +99,18 @@ int main() {
     CHECK(b.alloc(60) == PW_OK && b.alloc(90) == PW_OK && g_used == 90);
   }
   CHECK(g_used == 0);
+  {
+    // a batched reduction needs a place for every product
+    double x;
+    pwb::ReduceOut o;
+    o.out = &x;
+    CHECK(pwb::reduce_ok(o, 1) && !pwb::reduce_ok(o, 2));
+    o.out = nullptr;
+    o.bf_hi = &x;
+    CHECK(pwb::reduce_ok(o, 1) && !pwb::reduce_ok(o, 2));
+    o.bs_bf = 8;
+    CHECK(pwb::reduce_ok(o, 65535) && !pwb::reduce_ok(o, 65536) && !pwb::reduce_ok(o, 0));
+  }
   std::puts("ok");
   return 0;
 }
