@@ -63,8 +63,7 @@ template <int R, int M, int DIR, typename V> __device__ __forceinline__ V twmul(
 }
 
 template <int R> struct FirstFactor {
-  static constexpr int v = R == 30 ? 5                     // 5, 2, 3: the least rounding of its orders
-                         : (R % 4 == 0 && R != 4) ? 4
+  static constexpr int v = (R % 4 == 0 && R != 4) ? 4
                          : (R % 2 == 0 && R != 2) ? 2
                          : (R % 3 == 0 && R != 3) ? 3
                          : (R % 5 == 0 && R != 5) ? 5 : R;

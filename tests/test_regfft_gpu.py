@@ -66,3 +66,27 @@ def test_exchange_of_an_odd_number_of_orbitals(n, prec):
     kern = c.exx_kernel()[1][:, :, : n[0] // 2 + 1]
     ref = exx.add_mult_spinor_exx(T.dm, psi, exx.set_phi(T.dm, phi), kern, 0.25, occ)
     _close(c.exx_apply(torch.tensor(psi, dtype=c.torch_dtype, device="cuda")), ref, prec)
+
+
+@pytest.mark.parametrize("n", [(12, 12, 12), (16, 16, 16), (20, 20, 20), (24, 16, 20), (24, 24, 24), (30, 30, 30),
+                               (32, 32, 32), (36, 36, 36), (40, 40, 40), (48, 48, 48), (60, 60, 60), (72, 72, 72)])
+def test_rounding_of_the_transforms(n):
+    """FP32 Teter (a 3-D transform there and back) on damped bands: the rms error of
+    an FFT of N points grows as u sqrt(log2 N) (Gentleman and Sande 1966), here
+    with a factor of 0.36-0.49 over the lengths.  The bound of 0.52 leaves 5 % and is
+    passed by one more rounded twiddle product per point: with twiddles between all
+    radix steps 40 points are at 0.63, 36 at 0.56 and 72 at 0.521."""
+    import torch
+    c, T, _ = _case(n, "f32")
+    g = torch.Generator(device="cuda").manual_seed(5)
+    f = [2 * np.pi / (0.35 * m) * torch.fft.fftfreq(m, 1.0 / m, dtype=torch.float64, device="cuda") for m in n]
+    a = f[2][:, None, None] ** 2 + f[1][None, :, None] ** 2 + f[0][None, None, :] ** 2
+    b = 27.0 + a * (18.0 + a * (12.0 + a * 8.0))
+    x = torch.randn((16,) + n[::-1], generator=g, device="cuda", dtype=torch.float64)
+    x = torch.fft.ifftn(torch.fft.fftn(x, dim=(1, 2, 3)) / (1.0 + a / 6.0) ** 2, dim=(1, 2, 3)).real
+    x = x.reshape(16, -1).float()
+    ref = torch.fft.ifftn(torch.fft.fftn(x.double().reshape((16,) + n[::-1]), dim=(1, 2, 3)) * (b / (b + 16.0 * a ** 4)),
+                          dim=(1, 2, 3))
+    ref = ref.real.reshape(16, -1)
+    err = float((c.teter(x).double() - ref).norm() / ref.norm())
+    assert err <= 0.52 * 2.0 ** -24 * np.sqrt(2 * np.log2(c.ntot)), err
