@@ -409,13 +409,12 @@ typedef struct pw_tune_result {
   double ms_best;           /* sweep time with the chosen setting */
   int fft_variant;          /* H*psi transforms: 0 shared memory, 1 second radix split, 2 (default) registers */
 } pw_tune_result;
-/* Select the form of the fused fine-plane transforms directly (0: the first
- * radix decomposition N = n1 x n2 of each length with the inter-stage
- * twiddles read from shared-memory tables, 1: the second decomposition, e.g.
- * 96 = 12 x 8 instead of 8 x 12, 2 (the default): the first decomposition
- * with the twiddles of a transform formed in registers from one table entry
- * and the local potential read in the row pass's lane order); pw_autotune
- * times all three.  No reference counterpart. */
+/* Select the form of the H*psi transforms (dense projector mode and k-points;
+ * the sphere-cut mode takes it for its fine planes): 0 shared-memory passes with
+ * the first radix decomposition N = n1 x n2 of each length, 1 the same with the
+ * second decomposition in the fine planes, e.g. 96 = 12 x 8 instead of 8 x 12,
+ * 2 (the default) transforms in registers; pw_autotune times all three.  No
+ * reference counterpart. */
 PW_API int pw_set_fft_variant(pw_ctx* ctx, int variant);
 PW_API int pw_autotune(pw_ctx* ctx, int nband, pw_tune_result* result);
 

@@ -1,8 +1,8 @@
 // Autotuner for the H*psi sweep: times pw_hpsi on a scratch block (L2
 // flushed before each timed sweep) for candidate band-batch widths, the three
-// forms of the fused fine-plane transforms (two radix decompositions, and
-// register-formed twiddles) and, for FP32
-// contexts with projectors, the tile widths of the two projector GEMMs
+// forms of the transforms (in registers, and two radix decompositions in shared
+// memory) and, for FP32 contexts with projectors, the tile widths of the two
+// projector GEMMs
 // (coordinate descent; a candidate must beat the current best by 3%), keeps
 // the fastest setting in the context and caches it per (grid, precision,
 // bands, projectors) for later contexts of the same shape.
@@ -124,8 +124,7 @@ int pw_autotune(pw_ctx* ctx, int nband, pw_tune_result* res) {
     if ((rc = run(bb, 0, 0, &t))) return rc;
     if (t < 0.97 * best) { best = t; best_bb = bb; }
   }
-  // the other forms of the fine-plane transforms (dense projector mode: the
-  // fused fine-plane kernel)
+  // the shared-memory forms of the transforms (dense projector mode)
   int best_var = 2;
   if (ctx->nl_mode == PW_NL_DENSE && !ctx->gs) {
     for (int var : {0, 1}) {

@@ -295,10 +295,10 @@ struct Launch {
   }
 };
 
-// whether the projector products run beside the FFT chain.  At every size: even
-// where a call is shorter than its launches, the products of one call then run
-// under the chain of the call before (Al4 20^3, 7 bands, calls back to back:
-// 38 us, in one stream 50 us)
+// whether the projector products of a call run beside its FFT chain (where
+// pw_set_nl_overlap has it on: FP32 contexts by default, FP64 ones run them
+// after it).  At every size: the smallest calls gain too (Al4 20^3, 7 bands: 38 us,
+// in one stream 50 us)
 inline bool nl_beside_chain(const pw_ctx* c) {
   return c->nl_mode == PW_NL_DENSE && c->have_nl && c->nproj > 0 && c->nl_overlap && !c->prof_on;
 }

@@ -1372,7 +1372,8 @@ struct Plan {
     return sizeof(V) * ((size_t)floc_s_size<LY, NF1, NF1 / SplitVar<NF1, VAR>::n1>() + NF0 + NF1 +
                         (size_t)(FLOC_THREADS / 32) * (32 / SplitVar<NF0, VAR>::n1) * LY::PR);
   }
-  // the fused fine-plane kernel in the context's form
+  // the fused fine-plane kernel in the context's form (dual-grid contexts come
+  // here in the shared-memory forms 0 and 1 only)
   static void launch_floc2(pw_ctx* c, V* BC, const T* vt, T inv_nf, int nblk, cudaStream_t st) {
     if (c->fft_variant == 2 && c->gs)
       // sphere-cut slots are [ky][kx]: the axes and the potential change places
