@@ -351,3 +351,34 @@ def test_projector_builds_take_fields_for_their_projectors():
     d.set_kpoint(ks[1] / 2)
     x = y[0, :5].contiguous()
     assert torch.equal(c.hpsi_k(x), d.hpsi_k(x))
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("by", ["hpsi", "teter", "kbatch"])
+def test_a_captured_call_outlives_a_growth(by, prec):
+    """A graph recorded before wide H*psi, Teter or k-point calls grew the scratch
+    still reads and writes its own blocks."""
+    import torch
+    c = _ctx(prec)
+    x = _rand(c, 7)
+    out = torch.empty_like(x)
+    g = c.capture_hpsi(x, out)
+    g.replay()
+    torch.cuda.synchronize()
+    ref = out.clone()
+    if by == "kbatch":
+        c.set_kpoints(np.random.default_rng(1).uniform(-0.3, 0.3, (5, 3)))
+        r = torch.Generator(device="cuda").manual_seed(2)
+        big = torch.view_as_complex(torch.randn((5, 40, c.ntot, 2), generator=r, device="cuda", dtype=x.dtype))
+        f = c.hpsi_kbatch
+    else:
+        big = _rand(c, 200, seed=9)
+        f = c.hpsi if by == "hpsi" else c.teter
+    y = [f(big) for _ in range(3)]
+    assert all(torch.equal(v, y[0]) for v in y)
+    for _ in range(2):
+        out.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref)
+    assert torch.equal(f(big), y[0])
