@@ -421,7 +421,11 @@ PW_API int pw_autotune(pw_ctx* ctx, int nband, pw_tune_result* result);
 /* CUDA graph of one pw_hpsi call (same pointers, band count and accumulate
  * flag on every replay; the inputs' contents may change between replays).
  * The capture runs one ordinary call first (outside the graph).  Replays
- * issue every kernel and library GEMM of the sweep with one launch. */
+ * issue every kernel and library GEMM of the sweep with one launch.  The graph
+ * reads the context's scratch, which stays valid however wide later calls are,
+ * and its operator tables: new values of the potential are seen, but setting
+ * projectors, exchange orbitals or ACE vectors again, or destroying the context,
+ * ends its validity (capture again). */
 typedef struct pw_graph pw_graph;
 PW_API int pw_graph_capture_hpsi(pw_ctx* ctx, const void* psi, int ld, void* hpsi, int ldh, int nband,
                                  int accumulate, pw_graph** graph);
