@@ -1530,16 +1530,18 @@ struct Plan {
     if (c->exx_mode == PW_EXX_OFF) return PW_OK;
     if (c->exx_mode == PW_EXX_ACE)
       return c->ace_n == 0 ? PW_OK : dense_call(c, ace_set(c, filt), psi, ld, out, ldo, nband, st);
-    int rc;
-    if (c->gs) {
-      // 64 bands at a time: its full-grid workspaces go with the bands
-      for (int b0 = 0; b0 < nband; b0 += 64)
-        if ((rc = gs_exx_apply(c, psi + (long)b0 * ld, ld, std::min(64, nband - b0), out + (long)b0 * ldo, ldo, 1, st)))
-          return rc;
-      return PW_OK;
+    // 64 bands at a time: the sphere-cut workspaces go with the bands, and the pair
+    // fields of more bands leave room for few orbitals of each, whose short sums
+    // cost more than they save (160 x 128 pairs of 48^3, FP32: 9.9 ms together, 9.4 ms
+    // in 64s; 480 x 64 of 72^3: 121 and 62 ms)
+    for (int b0 = 0; b0 < nband; b0 += 64) {
+      const int nb = std::min(64, nband - b0);
+      const T* x = psi + (long)b0 * ld;
+      T* y = out + (long)b0 * ldo;
+      const int rc = c->gs ? gs_exx_apply(c, x, ld, nb, y, ldo, 1, st) : exx_apply(c, x, ld, nb, y, ldo, 1, st);
+      if (rc) return rc;
     }
-    rc = exx_apply(c, psi, ld, nband, out, ldo, 1, st);
-    if (rc || !filt) return rc;
+    if (c->gs || !filt) return PW_OK;
     // the pair-FFT exchange has no fused filter: one explicit P pass over the
     // output bands (the local, kinetic and projector parts are already in the
     // filtered space, and P is idempotent)

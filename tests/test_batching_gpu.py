@@ -382,3 +382,22 @@ def test_a_captured_call_outlives_a_growth(by, prec):
         torch.cuda.synchronize()
         assert torch.equal(out, ref)
     assert torch.equal(f(big), y[0])
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+def test_the_exchange_of_a_wide_call_takes_64_bands_at_a_time(prec):
+    """The pair fields' chunks, and with them the sums over the orbitals, do not
+    follow the width of an H*psi call: the bits of calls of 64 bands."""
+    import torch
+    from pwdft_develop_b200 import Context
+    from pwdft_develop_b200._lib import check, lib
+    c = Context((A,) * 3, (16, 16, 16), (32, 32, 32), precision=prec)
+    c.set_vtot(np.random.default_rng(3).uniform(-1, 0.5, c.ntotFine))
+    c.exx_setup(0.25, 0.0, 1, 6.0)
+    c.exx_set_phi(_rand(c, 30, seed=4) / np.sqrt(c.ntot), np.ones(30))
+    c.exx_set_mode("full")
+    x = _rand(c, 150) / np.sqrt(c.ntot)
+    # room for 256 pair fields: 4 orbital pairs of 64 bands, 1 of 150
+    check(lib.pw_exx_set_scratch(c.handle, 256 * c.ntot * (16 if prec == "f64" else 8)))
+    ref = torch.cat([c.hpsi(x[i:i + 64]) for i in range(0, 150, 64)])
+    assert torch.equal(c.hpsi(x), ref)
